@@ -1,5 +1,5 @@
 // engine.cu -- the C ABI of include/mhm_gpu.h: context, device memory, the
-// chunked time loop (cell chain -> L1->L11 accumulation -> level routing) and
+// chunked time loop (cell chain -> L1->L11 accumulation -> routing) and
 // state/variable access.
 #include <cuda_runtime.h>
 
@@ -29,8 +29,7 @@ cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
 cudaError_t launch_steps_fill(StepInfo *steps, int64_t tt0, int32_t n, int32_t jul_start, int32_t timestep,
                               int32_t stride, int32_t lai_mode, cudaStream_t s);
 cudaError_t launch_runoff_acc(const AccArgs &a, cudaStream_t s);
-cudaError_t launch_route_tick(const RouteArgs &a, cudaStream_t s);
-cudaError_t launch_route_walk(const RouteArgs &a, const RouteWalk &w, int cs, cudaStream_t s);
+cudaError_t launch_route_flow(const RouteArgs &a, int round, cudaStream_t s);
 cudaError_t launch_qmod_step(const QmodStepArgs &a, cudaStream_t s);
 cudaError_t launch_gauge_gather(const GaugeArgs &a, cudaStream_t s);
 cudaError_t launch_qrouted(const QroutArgs &a, cudaStream_t s);
@@ -100,25 +99,6 @@ struct OutSet {
     DevBuf<double> acc, out;
 };
 
-// The routing wavefront of one chunk (D + n_sub - 1 launches of
-// route_tick_kernel) captured once as a CUDA graph per argument set and
-// replayed for every chunk of that shape: the tick launches differ only in
-// tick / position range, which depend on the network and the chunk length.
-struct RouteGraph {
-    RouteArgs key{};
-    int32_t n_ticks = 0;
-    cudaGraphExec_t exec = nullptr;
-};
-
-bool same_route_shape(const RouteArgs &a, const RouteArgs &b)
-{
-    return a.n_nodes == b.n_nodes && a.n_members == b.n_members && a.n_steps == b.n_steps && a.sub == b.sub &&
-           a.rdiv == b.rdiv && a.n_qsteps == b.n_qsteps && a.pos_level == b.pos_level && a.up_ptr == b.up_ptr &&
-           a.up_pos == b.up_pos && a.pos_flags == b.pos_flags && a.C1 == b.C1 && a.C2 == b.C2 && a.qout == b.qout &&
-           a.qtr == b.qtr && a.qmod == b.qmod && a.qtin1 == b.qtin1 && a.qtr1 == b.qtr1 &&
-           a.member_step0 == b.member_step0;
-}
-
 struct ForcingSrc {
     const double *ptr = nullptr;
     int32_t row0 = 0, n_rows = 0, on_device = 0;
@@ -135,7 +115,7 @@ struct mhm_ctx {
     int device = 0;
     MonthTables tab{};
     double ss_max = 0.0;
-    LevelNetwork net;
+    RouteNetwork net;
     std::vector<int32_t> gauge_pos;
     std::vector<int32_t> link_to;    // [n_links] 0-based node each link drains into
     DevBuf<int32_t> nonfinite;       // [M] per-member non-finite flags of the cell chain
@@ -149,11 +129,21 @@ struct mhm_ctx {
     // device: static
     DevBuf<double> params, states, latitude, l1_area, pos_area, length, slope, ffp, rout_p5;
     DevBuf<double> C1, C2, qtin1, qtr1, qout_last, qmod_last;
-    DevBuf<int32_t> node_cell_ptr, node_cells, pos_l11_l1, up_ptr, up_pos, link_pos, gauge_pos_d, pos_level;
+    DevBuf<int32_t> node_cell_ptr, node_cells, pos_l11_l1, link_pos, gauge_pos_d;
     DevBuf<int8_t> pos_flags;
+    // routing blocks (RouteNetwork) and the series they hand over; the counters
+    // are never cleared: launches count on from the last one's
+    DevBuf<int32_t> blk_ptr, blk_lag, ext_ptr, ext_export, ext_lag, pos_lag, pos_export, hub_ptr, hub_ups;
+    DevBuf<int16_t> pos_ups;
+    DevBuf<uint32_t> route_words; // next (block, member), launch whose waits ran out
+    DevBuf<longlong2> qx;
+    uint32_t route_ticket0 = 0, route_launch = 1;
+    uint64_t route_done0 = 1;
+    int32_t route_polls = 1 << 22; // reads of one wait before it runs out (seconds)
+    int32_t *route_timed_out = nullptr; // host memory
     // device: per run / chunk
     DevBuf<StepInfo> steps;
-    DevBuf<double> tro[2], qout, qtr, qmod, q_gauge[2];
+    DevBuf<double> tro[2], qout, qmod, q_gauge[2];
     DevBuf<double> stage[kForcKinds][2];
     int32_t tc_cap = 0, stage_rows = 0;
     size_t qg_cap[2] = {0, 0};
@@ -196,13 +186,8 @@ struct mhm_ctx {
     int64_t t_launches[4] = {0, 0, 0, 0};
     double t_ms[4] = {0, 0, 0, 0};
     size_t chunk_bytes = (size_t)8 << 30;
-    int32_t route_sub = 8; // steps per wavefront sub-chunk (4, 8 or 16)
-    bool route_graphs_on = true;
-    std::vector<RouteGraph> route_graphs; // most recently used last
-    // 0: one launch per wavefront tick (replayed from a CUDA graph); 4, 8, 16:
-    // the whole wavefront of a chunk in one launch of clusters of that many CTAs
-    int32_t route_cluster = 0;
-    DevBuf<int32_t> level_ptr_d;
+    int32_t route_sub = 8;     // steps the routing fetches ahead at a time (1..16: 4, or 8 above 4)
+    int32_t route_cluster = 0; // accepted and reported; a chunk's routing is one launch either way
     // timeStep_LAI_input: 0 monthly LAI slots; -1 / -2 / -3 a gridded LAI series
     // of n_lai entries, its parameters in lai_series [M][3][n_lai][N]
     int32_t lai_mode = 0, n_lai = 0;
@@ -364,7 +349,7 @@ struct Bracket {
     }
 };
 
-// The routing stream gets the highest priority: its wavefront ticks are short,
+// The routing stream gets the highest priority: its blocks are short,
 // latency-bound launches that should take the next free SM slot ahead of the
 // cell-chain blocks they overlap with.
 cudaError_t route_stream_create(cudaStream_t *s)
@@ -399,6 +384,8 @@ static __device__ __align__(256) double g_mpr_scratch[kMprScratchDoubles];
 constexpr int kMaxScratchDevices = 64;
 static std::mutex g_scratch_mu;
 static double *g_scratch_addr[kMaxScratchDevices] = {};
+// rows of an exported outflow series: whole 128-byte lines
+static inline size_t qx_rows(size_t steps) { return (steps + 7) & ~(size_t)7; }
 static inline size_t align32(size_t n) { return (n + 31) & ~(size_t)31; } // 256-byte steps
 
 namespace {
@@ -521,7 +508,7 @@ int read_outset(mhm_ctx *ctx, OutSet &o, double *out, int64_t *slot_tt, int32_t 
     const size_t per = (size_t)o.n_planes * ctx->M * (by_node ? (size_t)ctx->L : (size_t)ctx->N);
     if (o.slots > 0)
         CK(cudaMemcpy(out, o.out.p, (size_t)o.slots * per * sizeof(double), cudaMemcpyDeviceToHost), "outputs");
-    if (by_node) { // routing-level positions -> L11 node order
+    if (by_node) { // routing positions -> L11 node order
         const size_t L = ctx->L;
         std::vector<double> row(L);
         for (size_t r = 0; r < (size_t)o.slots * ctx->M; ++r) {
@@ -611,17 +598,19 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
         ctx->n_out = d->n_outlets;
         std::string err;
         if (ctx->L > 1) {
-            if (!build_level_network(d->n_nodes, d->n_outlets, d->net_perm, d->from_n, d->to_n, ctx->net, err))
+            if (!build_route_network(d->n_nodes, d->n_outlets, d->net_perm, d->from_n, d->to_n, kRouteBlock,
+                                     ctx->net, err))
                 return bad(err);
         } else {
-            ctx->net = LevelNetwork{};
-            ctx->net.n_nodes = 1;
-            ctx->net.n_levels = 1;
-            ctx->net.level_ptr = {0, 1};
-            ctx->net.pos_of_node = {0};
-            ctx->net.node_of_pos = {0};
-            ctx->net.up_ptr = {0, 0};
+            ctx->net = RouteNetwork{};
+            ctx->net.n_nodes = ctx->net.n_blocks = 1;
+            ctx->net.pos_of_node = ctx->net.node_of_pos = ctx->net.blk_lag = ctx->net.pos_lag = {0};
             ctx->net.pos_flags = {2}; // Qmod = qOUT for a single node
+            ctx->net.blk_ptr = {0, 1};
+            ctx->net.ext_ptr = {0, 0};
+            ctx->net.pos_export = {-1};
+            ctx->net.pos_ups.assign(kRouteUps, -1);
+            ctx->net.hub_ptr = {0};
         }
         ctx->n_links = ctx->net.n_links;
         for (int i = 0; i < ctx->n_links; ++i) ctx->link_to.push_back(d->to_n[i] - 1);
@@ -632,6 +621,7 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
             int v = d->gauge_node[g] - 1;
             if (v < 0 || v >= ctx->L) return bad("gauge node out of range");
             ctx->gauge_pos.push_back(ctx->net.pos_of_node[v]);
+            ctx->net.pos_flags[ctx->gauge_pos.back()] |= 16; // its Qmod series is always written
         }
         for (int k = 0; k < ctx->N; ++k)
             if (d->l1_l11_id[k] < 1 || d->l1_l11_id[k] > ctx->L) return bad("L1_L11_Id out of range");
@@ -687,7 +677,7 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
     }
     if (ok && ctx->proc_pet == 1) ok = ck(upload(ctx->latitude, d->latitude, N, ctx->stream), "latitude");
     if (ok && ctx->proc_rout >= 1) {
-        const LevelNetwork &net = ctx->net;
+        const RouteNetwork &net = ctx->net;
         // L1 cells of each node in ascending cell order, by position
         std::vector<int32_t> cnt(L + 1, 0), cells(N);
         for (size_t k = 0; k < N; ++k) cnt[net.pos_of_node[d->l1_l11_id[k] - 1] + 1]++;
@@ -706,13 +696,19 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
         ok = ok && ck(upload(ctx->pos_l11_l1, pl1.data(), L, ctx->stream), "l11_l1");
         ok = ok && ck(upload(ctx->pos_area, parea.data(), L, ctx->stream), "l11 area");
         if (d->map_flag) ok = ok && ck(upload(ctx->l1_area, d->l1_area_km2, N, ctx->stream), "l1 area");
-        std::vector<int32_t> plev(L, 0);
-        for (int l = 0; l < net.n_levels; ++l)
-            for (int p = net.level_ptr[l]; p < net.level_ptr[l + 1]; ++p) plev[p] = l;
-        ok = ok && ck(upload(ctx->pos_level, plev.data(), L, ctx->stream), "levels");
-        ok = ok && ck(upload(ctx->level_ptr_d, net.level_ptr.data(), net.level_ptr.size(), ctx->stream), "level ptr");
-        ok = ok && ck(upload(ctx->up_ptr, net.up_ptr.data(), L + 1, ctx->stream), "up ptr");
-        ok = ok && ck(upload(ctx->up_pos, net.up_pos.data(), net.up_pos.size(), ctx->stream), "up pos");
+        const std::pair<DevBuf<int32_t> *, const std::vector<int32_t> *> tables[] = {
+            {&ctx->blk_ptr, &net.blk_ptr},       {&ctx->blk_lag, &net.blk_lag}, {&ctx->ext_ptr, &net.ext_ptr},
+            {&ctx->ext_export, &net.ext_export}, {&ctx->ext_lag, &net.ext_lag}, {&ctx->pos_lag, &net.pos_lag},
+            {&ctx->pos_export, &net.pos_export}, {&ctx->hub_ptr, &net.hub_ptr}, {&ctx->hub_ups, &net.hub_ups}};
+        for (const auto &t : tables)
+            ok = ok && ck(upload(*t.first, t.second->data(), t.second->size(), ctx->stream), "routing blocks");
+        ok = ok && ck(upload(ctx->pos_ups, net.pos_ups.data(), net.pos_ups.size(), ctx->stream), "routing blocks");
+        ok = ok && ck(ctx->route_words.ensure(2), "routing counters");
+        ok = ok && ck(cudaMallocHost((void **)&ctx->route_timed_out, sizeof(int32_t)), "routing status");
+        if (ok) {
+            *ctx->route_timed_out = 0;
+            cudaMemsetAsync(ctx->route_words.p, 0, 2 * sizeof(uint32_t), ctx->stream);
+        }
         ok = ok && ck(upload(ctx->pos_flags, net.pos_flags.data(), L, ctx->stream), "flags");
         ok = ok && ck(upload(ctx->link_pos, net.link_pos.data(), net.link_pos.size(), ctx->stream), "link pos");
         ok = ok && ck(upload(ctx->gauge_pos_d, ctx->gauge_pos.data(), ctx->gauge_pos.size(), ctx->stream), "gauges");
@@ -746,7 +742,7 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
         int v = std::atoi(s);
         if (v == 4 || v == 6 || v == 8) ctx->cell_occ = v;
     }
-    if (const char *s = std::getenv("MHM_ROUTE_GRAPH")) ctx->route_graphs_on = std::atoi(s) != 0;
+    if (const char *s = std::getenv("MHM_ROUTE_POLLS")) ctx->route_polls = std::max(0, std::atoi(s));
     if (const char *s = std::getenv("MHM_ROUTE_CLUSTER")) {
         int v = std::atoi(s);
         if (v == 0 || v == 4 || v == 8 || v == 16) ctx->route_cluster = v;
@@ -779,8 +775,7 @@ int mhm_ctx_destroy(mhm_ctx *ctx)
     for (cudaEvent_t e : ctx->ev_members_done)
         if (e) cudaEventDestroy(e);
     if (ctx->run_a) cudaEventDestroy(ctx->run_a);
-    for (auto &rg : ctx->route_graphs)
-        if (rg.exec) cudaGraphExecDestroy(rg.exec);
+    if (ctx->route_timed_out) cudaFreeHost(ctx->route_timed_out);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->route_stream) cudaStreamDestroy(ctx->route_stream);
@@ -1284,7 +1279,6 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         for (int s = 0; s < 2; ++s) CK(ctx->tro[s].ensure((size_t)Tc * M * N), "total runoff chunk");
         if (ctx->proc_rout >= 1) {
             CK(ctx->qout.ensure(M * (size_t)Tc * L), "qout chunk");
-            CK(ctx->qtr.ensure(M * (size_t)Tc * L), "qtr chunk");
             CK(ctx->qmod.ensure(M * (size_t)Tc * L), "qmod chunk");
         }
         const int32_t max_rows = (Tc + stride - 1) / stride + 1;
@@ -1295,10 +1289,17 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
     }
     if ((R > 1 || F > 1) && ctx->proc_rout >= 1) {
         const size_t need_rt = M * (size_t)ctx->tc_cap * R * L;
-        if (ctx->qtr.n < need_rt || ctx->qmod_sub.n < need_rt) {
+        if (ctx->qmod_sub.n < need_rt) {
             CK(cudaStreamSynchronize(ctx->route_stream), "sync");
-            CK(ctx->qtr.ensure(need_rt), "qtr routing steps");
             CK(ctx->qmod_sub.ensure(need_rt), "qmod routing steps");
+        }
+    }
+    if (ctx->proc_rout >= 1) {
+        const size_t need_x = M * ctx->net.n_exports * qx_rows((size_t)ctx->tc_cap * R);
+        if (ctx->qx.n < need_x) {
+            CK(cudaStreamSynchronize(ctx->route_stream), "sync");
+            CK(ctx->qx.ensure(need_x), "routed outflow series");
+            CK(cudaMemsetAsync(ctx->qx.p, 0, need_x * sizeof(longlong2), ctx->route_stream), "routed outflow series");
         }
     }
     if (!on_device)
@@ -1576,79 +1577,49 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         r.n_steps = n_rsteps;
         r.rdiv = R;
         r.n_qsteps = nT / F;
-        r.sub = std::min(ctx->route_sub, n_rsteps);
-        r.pos_level = ctx->pos_level.p;
-        r.up_ptr = ctx->up_ptr.p;
-        r.up_pos = ctx->up_pos.p;
+        r.n_blocks = ctx->net.n_blocks;
+        r.n_exports = ctx->net.n_exports;
+        r.blk_ptr = ctx->blk_ptr.p;
+        r.blk_lag = ctx->blk_lag.p;
+        r.ext_ptr = ctx->ext_ptr.p;
+        r.ext_export = ctx->ext_export.p;
+        r.ext_lag = ctx->ext_lag.p;
+        r.pos_lag = ctx->pos_lag.p;
+        r.pos_export = ctx->pos_export.p;
+        r.hub_ptr = ctx->hub_ptr.p;
+        r.hub_ups = ctx->hub_ups.p;
+        r.pos_ups = ctx->pos_ups.p;
         r.pos_flags = ctx->pos_flags.p;
         r.C1 = ctx->C1.p;
         r.C2 = ctx->C2.p;
         r.qout = ctx->qout.p;
-        r.qtr = ctx->qtr.p;
+        r.qx = ctx->qx.p;
+        r.qx_stride = (int64_t)qx_rows((size_t)ctx->tc_cap * R);
         r.qmod = (R > 1 || F > 1) ? ctx->qmod_sub.p : ctx->qmod.p;
+        r.qmod_all = R > 1 || F > 1 || ctx->out_qmod || ctx->qro.on;
         r.qtin1 = ctx->qtin1.p;
         r.qtr1 = ctx->qtr1.p;
+        // the restart fields of the chunk's last step, unless they are written
+        // below (Qrouted still reads the previous chunk's Qmod; with several
+        // routing passes a step Qmod is their mean)
+        const bool last_here = R == 1 && !ctx->qro.on;
+        r.qout_last = last_here ? ctx->qout_last.p : nullptr;
+        r.qmod_last = last_here ? ctx->qmod_last.p : nullptr;
         r.member_step0 = members ? ctx->member_s0_cur : nullptr;
+        r.ticket = ctx->route_words.p;
+        r.abort = ctx->route_words.p + 1;
+        r.ticket0 = ctx->route_ticket0;
+        r.done0 = ctx->route_done0;
+        r.launch = ctx->route_launch;
+        r.max_polls = ctx->route_polls;
+        r.timed_out = ctx->route_timed_out;
         {
             Bracket br(ctx, 2, rs);
-            // wavefront: tick k advances sub-chunk k - l of level l
-            const int D = ctx->net.n_levels;
-            const int n_sub = (n_rsteps + r.sub - 1) / r.sub;
-            const int n_ticks = D + n_sub - 1;
-            auto enqueue_ticks = [&]() -> int {
-                if (ctx->route_cluster > 0) { // all ticks in one launch
-                    RouteWalk w{};
-                    w.level_ptr = ctx->level_ptr_d.p;
-                    w.n_levels = D;
-                    w.n_sub = n_sub;
-                    w.n_ticks = n_ticks;
-                    CK(launch_route_walk(r, w, ctx->route_cluster, rs), "route walk launch");
-                    return MHM_OK;
-                }
-                for (int k = 0; k < n_ticks; ++k) {
-                    const int lo = std::max(0, k - n_sub + 1), hi = std::min(k, D - 1);
-                    r.tick = k;
-                    r.pos_begin = ctx->net.level_ptr[lo];
-                    r.pos_end = ctx->net.level_ptr[hi + 1];
-                    CK(launch_route_tick(r, rs), "route launch");
-                }
-                return MHM_OK;
-            };
-            if (ctx->route_graphs_on && ctx->route_cluster == 0) {
-                auto &cache = ctx->route_graphs;
-                auto it = std::find_if(cache.begin(), cache.end(),
-                                       [&](const RouteGraph &g) { return same_route_shape(g.key, r); });
-                if (it == cache.end()) {
-                    RouteGraph rg;
-                    rg.key = r;
-                    rg.n_ticks = n_ticks;
-                    cudaGraph_t graph = nullptr;
-                    CK(cudaStreamBeginCapture(rs, cudaStreamCaptureModeThreadLocal), "route capture");
-                    const int rc_cap = enqueue_ticks();
-                    const cudaError_t e_end = cudaStreamEndCapture(rs, &graph);
-                    if (rc_cap) {
-                        if (graph) cudaGraphDestroy(graph);
-                        return rc_cap;
-                    }
-                    CK(e_end, "route capture end");
-                    const cudaError_t e_inst = cudaGraphInstantiate(&rg.exec, graph, 0);
-                    cudaGraphDestroy(graph);
-                    CK(e_inst, "route graph instantiate");
-                    if (cache.size() >= 8) { // keep the most recently used shapes
-                        cudaGraphExecDestroy(cache.front().exec);
-                        cache.erase(cache.begin());
-                    }
-                    cache.push_back(rg);
-                    it = cache.end() - 1;
-                } else if (it != cache.end() - 1) {
-                    std::rotate(it, it + 1, cache.end());
-                    it = cache.end() - 1;
-                }
-                CK(cudaGraphLaunch(it->exec, rs), "route graph launch");
-            } else if (int rc = enqueue_ticks()) {
-                return rc;
-            }
-            g_launches += ctx->route_cluster > 0 ? 1 : n_ticks;
+            CK(launch_route_flow(r, ctx->route_sub, rs), "route launch");
+            ctx->route_ticket0 += (uint32_t)(r.n_blocks * r.n_members);
+            ctx->route_done0 += (uint64_t)n_rsteps;
+            ctx->route_launch += 1;
+            g_launches++;
             if (R > 1 || F > 1) {
                 QmodStepArgs qs{};
                 qs.n_members = ctx->M;
@@ -1707,7 +1678,7 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
             g_launches++;
             out_advance(ctx->qro, ctx->jul_start, ctx->timestep, (int64_t)tt0 + s0, nT, true);
         }
-        if (c == nchunks - 1 || ctx->qro.on) {
+        if (!last_here && (c == nchunks - 1 || ctx->qro.on)) {
             // qOUT and Qmod of the chunk's last step (restart fields; the
             // Qrouted output of the next chunk starts from this Qmod)
             for (size_t m = 0; m < M; ++m) {
@@ -1843,8 +1814,12 @@ int mhm_sync(mhm_ctx *ctx)
     for (auto &st : ctx->qg_stage)
         if (int rc = finish_gauge_stage(ctx, st)) return rc;
     harvest_timing(ctx);
+    if (ctx->route_timed_out && *ctx->route_timed_out) {
+        *ctx->route_timed_out = 0;
+        return fail(ctx, MHM_ERR_TIMEOUT, "a wait of the routing kernel ran out");
+    }
     if (int rc = take_bounds_status(ctx, nullptr, nullptr)) return rc;
-    if (ctx->pending_outputs && ctx->out_qmod) { // routing-level positions -> node order
+    if (ctx->pending_outputs && ctx->out_qmod) { // routing positions -> node order
         const size_t L = ctx->L;
         std::vector<double> row(L);
         for (size_t r = 0; r < (size_t)ctx->M * (size_t)ctx->last_steps; ++r) {
@@ -2052,8 +2027,7 @@ int mhm_autotune_ex(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t n_chunk_
     float best = 1e30f;
     int best_occ = occ0, best_sub = sub0, best_cap = cap0;
     // untimed warm-ups first, so that no timed trial pays a first use: module
-    // loading of each kernel variant and the capture of each routing graph
-    // (every routing sub-chunk with every chunk length)
+    // loading of each kernel variant and buffers of each chunk length
     std::vector<int> warm;
     for (int c = 0; c < nc; ++c)
         for (int j = 0; j < 3; ++j) warm.push_back(c * 9 + j);     // (4, sub) for each chunk length

@@ -3,6 +3,8 @@
 #pragma once
 #include <cstdint>
 
+#include <vector_types.h>
+
 namespace mhm {
 
 constexpr int kMaxHorizons = 8;
@@ -179,36 +181,38 @@ struct AccArgs {
     const int32_t *member_step0;  // member mode: < 0 marks an idle member (skipped)
 };
 
-// Wavefront routing: the chunk is cut into sub-chunks of `sub` steps; launch
-// `tick` advances sub-chunk (tick - level) of every node whose level is in
-// [lvl_lo, lvl_hi] (positions pos_begin .. pos_end-1).
+// Routing of a chunk in one launch (route_flow_kernel): the network's blocks
+// (RouteNetwork in network.h) times the members.
 struct RouteArgs {
     int32_t n_nodes, n_members, n_steps;
-    int32_t pos_begin, pos_end;
-    int32_t tick, sub;
-    const int32_t *pos_level;   // [n_nodes] topological level of each position
-    const int32_t *up_ptr;      // [n_nodes+1]
-    const int32_t *up_pos;      // upstream positions in rank order
+    int32_t n_blocks, n_exports;
+    const int32_t *blk_ptr, *blk_lag, *ext_ptr, *ext_export, *ext_lag, *pos_lag, *pos_export, *hub_ptr, *hub_ups;
+    const int16_t *pos_ups;     // [n_nodes][kRouteUps]
     const int8_t *pos_flags;    // bit0: is link (has C1/C2), bit1: add qOUT, bit2: the link's routed
-                                // outflow is cut (it drains into a non-headwater inflow gauge's node)
+                                // outflow is cut (it drains into a non-headwater inflow gauge's node),
+                                // bit4: a gauge's node
     const double *C1, *C2;      // [M][n_nodes] by position
     // routing step s reads qOUT row s / rdiv of [M][n_qsteps][n_nodes]: with an
     // adaptive routing step shorter than the model step the model step's qOUT
     // is routed rdiv times
     int32_t rdiv, n_qsteps;
     const double *qout;
-    double *qtr;                // [M][n_steps][n_nodes] routed outflow series
-    double *qmod;               // [M][n_steps][n_nodes] (if write_qmod)
+    longlong2 *qx;              // [M][n_exports][qx_stride] exported outflow series (value, step number)
+    int64_t qx_stride;
+    double *qmod;               // [M][n_steps][n_nodes]: all nodes, or the gauges' only
+    int32_t qmod_all;
     double *qtin1, *qtr1;       // [M][n_nodes] state (previous step)
+    double *qout_last, *qmod_last; // [M][n_nodes] last row of qOUT / Qmod, or null
     const int32_t *member_step0; // member mode: < 0 marks an idle member (skipped)
-};
-
-// The wavefront of a chunk walked in one launch (route_walk_kernel): tick k
-// spans levels max(0, k - n_sub + 1) .. min(k, n_levels - 1), i.e. positions
-// level_ptr[lo] .. level_ptr[hi + 1] - 1.
-struct RouteWalk {
-    const int32_t *level_ptr; // [n_levels + 1] first routing position of each level
-    int32_t n_levels, n_sub, n_ticks;
+    // the next (block, member) to take, counted on from ticket0; step t of an
+    // exported series has the number done0 + t: nothing is cleared between launches
+    uint32_t *ticket;
+    uint32_t ticket0;
+    uint64_t done0;
+    uint32_t *abort;            // launch whose waits ran out
+    uint32_t launch;
+    int32_t max_polls;
+    int32_t *timed_out;         // host memory, set when a wait ran out
 };
 
 // add_inflow (src/mRM/mo_mrm_pre_routing.f90:179-214) on a chunk's qOUT rows,

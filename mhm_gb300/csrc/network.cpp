@@ -1,4 +1,4 @@
-// network.cpp -- routing-level layout and routing order (host).
+// network.cpp -- routing blocks and routing order (host).
 #include "network.h"
 
 #include <algorithm>
@@ -6,18 +6,19 @@
 
 namespace mhm {
 
-bool build_level_network(int32_t L, int32_t n_outlets, const int32_t *net_perm, const int32_t *from_n,
-                         const int32_t *to_n, LevelNetwork &o, std::string &err)
+bool build_route_network(int32_t L, int32_t n_outlets, const int32_t *net_perm, const int32_t *from_n,
+                         const int32_t *to_n, int32_t cap, RouteNetwork &o, std::string &err)
 {
-    o = LevelNetwork{};
+    o = RouteNetwork{};
     if (L < 1 || n_outlets < 1 || n_outlets > L) {
         err = "network: need n_nodes >= 1 and 1 <= n_outlets <= n_nodes";
         return false;
     }
+    cap = std::max(kRouteUps, std::min(cap, kRouteBlock));
     const int32_t nl = L - n_outlets;
     o.n_nodes = L;
     o.n_links = nl;
-    std::vector<int32_t> rank(nl, -1), out_link(L, -1);
+    std::vector<int32_t> rank(nl, -1), down(L, -1);
     for (int32_t r = 0; r < nl; ++r) {
         const int32_t i = net_perm[r] - 1;
         if (i < 0 || i >= nl || rank[i] != -1) {
@@ -32,60 +33,187 @@ bool build_level_network(int32_t L, int32_t n_outlets, const int32_t *net_perm, 
             err = "network: fromN/toN out of range or self loop";
             return false;
         }
-        if (out_link[f] != -1) {
+        if (down[f] != -1) {
             err = "network: a node is the source of two links";
             return false;
         }
-        out_link[f] = i;
+        down[f] = t;
     }
-    // upstream links per node, in rank order
+    // upstream nodes of each node in rank order of their links, and the nodes
+    // in rank order of their own link (sinks last): upstream before downstream
     std::vector<std::vector<int32_t>> ups(L);
+    std::vector<int32_t> topo, topo_of(L, -1);
     for (int32_t r = 0; r < nl; ++r) {
-        const int32_t i = net_perm[r] - 1;
-        ups[to_n[i] - 1].push_back(i);
+        const int32_t i = net_perm[r] - 1, f = from_n[i] - 1;
+        ups[to_n[i] - 1].push_back(f);
+        topo_of[f] = (int32_t)topo.size();
+        topo.push_back(f);
     }
-    // topological check: every upstream link of fromN(i) precedes i
-    for (int32_t i = 0; i < nl; ++i)
-        for (int32_t j : ups[from_n[i] - 1])
-            if (rank[j] >= rank[i]) {
+    for (int32_t v = 0; v < L; ++v)
+        if (down[v] < 0) {
+            topo_of[v] = (int32_t)topo.size();
+            topo.push_back(v);
+        }
+    for (int32_t v = 0; v < L; ++v)
+        for (int32_t u : ups[v])
+            if (topo_of[u] >= topo_of[v]) {
                 err = "network: netPerm is not a topological order of the links";
                 return false;
             }
-    // levels (longest path from a headwater), relaxed in rank order
-    std::vector<int32_t> level(L, 0);
-    for (int32_t r = 0; r < nl; ++r) {
-        const int32_t i = net_perm[r] - 1;
-        const int32_t f = from_n[i] - 1, t = to_n[i] - 1;
-        level[t] = std::max(level[t], level[f] + 1);
-    }
     const int32_t special_outlet = (nl > 0) ? to_n[net_perm[nl - 1] - 1] - 1 : -1;
-    // positions: by level, then by rank of the node's link (sinks last)
-    std::vector<int32_t> order(L);
+
+    // trunk: nodes whose subtree holds more than `cap` nodes or a hub (a node
+    // with more than kRouteUps upstream links); what is left are subtrees of
+    // at most `cap` nodes
+    std::vector<int32_t> size(L, 1);
+    std::vector<uint8_t> hub(L, 0), trunk(L, 0);
+    for (int32_t v : topo) {
+        hub[v] = (int32_t)ups[v].size() > kRouteUps;
+        for (int32_t u : ups[v]) {
+            size[v] += size[u];
+            trunk[v] |= trunk[u];
+        }
+        trunk[v] |= hub[v] || size[v] > cap;
+    }
+    // pieces: piece[v], a piece's nodes upstream first; `level` 0 for whole
+    // subtrees, for a stretch of the trunk one more than any piece draining into it
+    struct Piece {
+        std::vector<int32_t> nodes;
+        int32_t n_ext = 0, level = 0;
+    };
+    std::vector<Piece> pieces;
+    std::vector<int32_t> piece(L, -1);
+    for (size_t k = topo.size(); k-- > 0;) { // downstream first: a subtree's root opens its piece
+        const int32_t v = topo[k];
+        if (trunk[v]) continue;
+        if (down[v] >= 0 && !trunk[down[v]]) {
+            piece[v] = piece[down[v]];
+        } else {
+            piece[v] = (int32_t)pieces.size();
+            pieces.emplace_back();
+        }
+    }
+    for (int32_t v : topo)
+        if (!trunk[v]) pieces[piece[v]].nodes.push_back(v);
+    // trunk: every node continues the stretch of its longest upstream trunk
+    // branch until the stretch is full; all other links are cut
+    std::vector<int32_t> height(L, 0);
+    for (int32_t v : topo) {
+        if (!trunk[v]) continue;
+        int32_t main = -1;
+        for (int32_t u : ups[v])
+            if (trunk[u] && (main < 0 || height[u] > height[main])) main = u;
+        height[v] = main < 0 ? 1 : height[main] + 1;
+        const int32_t n_cut = (int32_t)ups[v].size() - (main >= 0 ? 1 : 0);
+        int32_t p = main >= 0 ? piece[main] : -1;
+        if (hub[v] || p < 0 || (int32_t)pieces[p].nodes.size() >= cap || pieces[p].n_ext + n_cut > cap) {
+            p = (int32_t)pieces.size();
+            pieces.emplace_back();
+            if (!hub[v]) pieces[p].n_ext = (int32_t)ups[v].size();
+        } else {
+            pieces[p].n_ext += n_cut;
+        }
+        piece[v] = p;
+        pieces[p].nodes.push_back(v);
+    }
+    std::vector<int32_t> order(pieces.size());
     std::iota(order.begin(), order.end(), 0);
-    auto key = [&](int32_t v) { return out_link[v] >= 0 ? (int64_t)rank[out_link[v]] : (int64_t)nl + v; };
+    auto last = [&](int32_t p) { return topo_of[pieces[p].nodes.back()]; };
+    std::sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return last(a) < last(b); });
+    for (int32_t p : order)
+        for (int32_t v : pieces[p].nodes)
+            for (int32_t u : ups[v])
+                if (piece[u] != p) pieces[p].level = std::max(pieces[p].level, pieces[piece[u]].level + 1);
+    // blocks: pieces of one level, filled in the order of the place they drain into
+    auto drains_to = [&](int32_t p) {
+        const int32_t d = down[pieces[p].nodes.back()];
+        return d < 0 ? L : topo_of[d];
+    };
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-        if (level[a] != level[b]) return level[a] < level[b];
-        return key(a) < key(b);
+        if (pieces[a].level != pieces[b].level) return pieces[a].level < pieces[b].level;
+        return drains_to(a) < drains_to(b);
     });
-    o.node_of_pos = order;
+    std::vector<std::vector<int32_t>> blocks;
+    int32_t fill = 0, fill_ext = 0, blk_level = -1;
+    for (int32_t p : order) {
+        const int32_t n = (int32_t)pieces[p].nodes.size(), e = pieces[p].n_ext;
+        if (pieces[p].level != blk_level || fill + n > cap || fill_ext + e > cap) {
+            blocks.emplace_back();
+            fill = fill_ext = 0;
+            blk_level = pieces[p].level;
+        }
+        fill += n;
+        fill_ext += e;
+        blocks.back().push_back(p);
+    }
+    // lags: the distance to the piece's last node, counted back from the piece's
+    // longest, so that a link inside a piece is always one tick
+    std::vector<int32_t> lag(L, 0), pos_in(L, 0);
+    for (const Piece &pc : pieces) {
+        int32_t deepest = 0;
+        for (size_t k = pc.nodes.size(); k-- > 0;) {
+            const int32_t v = pc.nodes[k];
+            lag[v] = k + 1 == pc.nodes.size() ? 0 : lag[down[v]] + 1;
+            deepest = std::max(deepest, lag[v]);
+        }
+        for (int32_t v : pc.nodes) lag[v] = deepest - lag[v];
+    }
+    o.n_blocks = (int32_t)blocks.size();
     o.pos_of_node.assign(L, 0);
-    for (int32_t p = 0; p < L; ++p) o.pos_of_node[order[p]] = p;
-    o.n_levels = level[order[L - 1]] + 1;
-    o.level_ptr.assign(o.n_levels + 1, 0);
-    for (int32_t v = 0; v < L; ++v) o.level_ptr[level[v] + 1]++;
-    for (int32_t l = 0; l < o.n_levels; ++l) o.level_ptr[l + 1] += o.level_ptr[l];
-    for (int32_t l = 0; l < o.n_levels; ++l)
-        o.max_width = std::max(o.max_width, o.level_ptr[l + 1] - o.level_ptr[l]);
-    o.up_ptr.assign(L + 1, 0);
+    o.node_of_pos.reserve(L);
+    o.pos_export.assign(L, -1);
+    o.blk_ptr.push_back(0);
+    std::vector<int32_t> export_of(L, -1);
+    for (const auto &blk : blocks) {
+        std::vector<int32_t> nodes;
+        for (int32_t p : blk) nodes.insert(nodes.end(), pieces[p].nodes.begin(), pieces[p].nodes.end());
+        // by lag: neighbouring threads work on the same step
+        std::stable_sort(nodes.begin(), nodes.end(), [&](int32_t a, int32_t b) { return lag[a] < lag[b]; });
+        for (size_t k = 0; k < nodes.size(); ++k) {
+            const int32_t v = nodes[k], pos = (int32_t)o.node_of_pos.size();
+            pos_in[v] = (int32_t)k;
+            o.pos_of_node[v] = pos;
+            o.node_of_pos.push_back(v);
+            if (down[v] >= 0 && piece[down[v]] != piece[v]) o.pos_export[pos] = export_of[v] = o.n_exports++;
+        }
+        o.blk_ptr.push_back((int32_t)o.node_of_pos.size());
+        o.blk_lag.push_back(lag[nodes.back()]);
+    }
+    o.ext_ptr.push_back(0);
+    o.pos_ups.assign((size_t)L * kRouteUps, -1);
     o.pos_flags.assign(L, 0);
-    for (int32_t p = 0; p < L; ++p) {
-        const int32_t v = order[p];
-        o.up_ptr[p + 1] = o.up_ptr[p] + (int32_t)ups[v].size();
-        for (int32_t j : ups[v]) o.up_pos.push_back(o.pos_of_node[from_n[j] - 1]);
-        int8_t fl = 0;
-        if (out_link[v] >= 0) fl |= 3; // a link adds its own qOUT (mo_mrm_routing.f90:445)
-        if (v == special_outlet) fl |= 2; // mo_mrm_routing.f90:466-467
-        o.pos_flags[p] = fl;
+    o.pos_lag.resize(L);
+    o.hub_ptr.push_back(0);
+    for (int32_t b = 0; b < o.n_blocks; ++b) {
+        for (int32_t pos = o.blk_ptr[b]; pos < o.blk_ptr[b + 1]; ++pos) {
+            const int32_t v = o.node_of_pos[pos];
+            o.pos_lag[pos] = lag[v];
+            int16_t *up = &o.pos_ups[(size_t)pos * kRouteUps];
+            if (hub[v]) {
+                const int32_t h = (int32_t)o.hub_ptr.size() - 1;
+                up[0] = -2;
+                up[1] = (int16_t)(h & 0x7fff);
+                up[2] = (int16_t)(h >> 15);
+                for (int32_t u : ups[v]) o.hub_ups.push_back(export_of[u]);
+                o.hub_ptr.push_back((int32_t)o.hub_ups.size());
+            } else {
+                int j = 0;
+                for (int32_t u : ups[v]) {
+                    if (piece[u] == piece[v]) {
+                        up[j++] = (int16_t)pos_in[u];
+                    } else {
+                        up[j++] = (int16_t)(kRouteBlock + (int32_t)o.ext_export.size() - o.ext_ptr[b]);
+                        o.ext_export.push_back(export_of[u]);
+                        o.ext_lag.push_back(lag[v]);
+                    }
+                }
+            }
+            int8_t fl = 0;
+            if (down[v] >= 0) fl |= 3; // a link adds its own qOUT (mo_mrm_routing.f90:445)
+            if (v == special_outlet) fl |= 2; // mo_mrm_routing.f90:466-467
+            o.pos_flags[pos] = fl;
+        }
+        o.ext_ptr.push_back((int32_t)o.ext_export.size());
     }
     o.link_pos.assign(nl, 0);
     for (int32_t i = 0; i < nl; ++i) o.link_pos[i] = o.pos_of_node[from_n[i] - 1];

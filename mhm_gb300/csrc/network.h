@@ -1,5 +1,6 @@
 // network.h -- host-side preparation of an L11 routing network for the
-// level-synchronous device routing, and the model-step calendar.
+// device routing (blocks of nodes that pass their outflow on), and the
+// model-step calendar.
 #pragma once
 #include <cstdint>
 #include <string>
@@ -7,27 +8,49 @@
 
 namespace mhm {
 
-// Routing network laid out by topological level (positions 0..n_nodes-1).
-struct LevelNetwork {
-    int32_t n_nodes = 0, n_links = 0, n_levels = 0;
-    std::vector<int32_t> level_ptr;  // [n_levels + 1] position ranges
-    std::vector<int32_t> pos_of_node; // [n_nodes] 0-based node -> position
-    std::vector<int32_t> node_of_pos; // [n_nodes]
-    std::vector<int32_t> up_ptr;      // [n_nodes + 1] by position
-    std::vector<int32_t> up_pos;      // upstream positions, netPerm rank order
-    std::vector<int8_t> pos_flags;    // bit0 is link, bit1 adds its own qOUT
-    std::vector<int32_t> link_pos;    // [n_links] 1-based link i-1 -> position of fromN(i)
-    int32_t max_width = 0;
+// Upstream links a routing thread takes from its block's shared memory; a node
+// with more of them (none on a D8 grid) reads them from device memory.
+constexpr int kRouteUps = 8;
+// Most nodes of a routing block, and most series it takes from other blocks.
+constexpr int kRouteBlock = 64;
+
+// The routing network cut into blocks of at most `cap` nodes, and the order of
+// the nodes on the device (positions 0..n_nodes-1, block by block).  A block is
+// one or several pieces -- whole subtrees near the headwaters, stretches of a
+// river further down -- whose nodes run one step behind the node upstream:
+// thread i of the block handles its position at `lag` ticks.  A piece leaves
+// the block only through its last node, whose outflow series is exported; the
+// blocks are in an order in which every exported series comes from an earlier
+// block than the one that reads it.
+struct RouteNetwork {
+    int32_t n_nodes = 0, n_links = 0;
+    int32_t n_blocks = 0, n_exports = 0;
+    std::vector<int32_t> pos_of_node;  // [n_nodes] 0-based node -> position
+    std::vector<int32_t> node_of_pos;  // [n_nodes]
+    std::vector<int8_t> pos_flags;     // bit0 is link, bit1 adds its own qOUT
+    std::vector<int32_t> link_pos;     // [n_links] 1-based link i-1 -> position of fromN(i)
+    std::vector<int32_t> blk_ptr;      // [n_blocks + 1] positions of a block
+    std::vector<int32_t> blk_lag;      // [n_blocks] largest lag of a block
+    std::vector<int32_t> ext_ptr;      // [n_blocks + 1] series a block takes from others
+    std::vector<int32_t> ext_export;   // their export index
+    std::vector<int32_t> ext_lag;      // the lag of the node that reads the series
+    std::vector<int32_t> pos_lag;      // [n_nodes]
+    std::vector<int32_t> pos_export;   // [n_nodes] export index of the node's outflow, -1: stays in the block
+    // [n_nodes][kRouteUps] upstream links in netPerm rank order: a thread of the
+    // block, kRouteBlock + a series of the block's list, or -1 past the last;
+    // [0] == -2: a node with more, export indexes hub_ups[hub_ptr[h]..], h = [1] + ([2] << 15)
+    std::vector<int16_t> pos_ups;
+    std::vector<int32_t> hub_ptr, hub_ups;
 };
 
-// Builds the level layout from L11_netPerm / L11_fromN / L11_toN (1-based, as
-// produced by L11_set_network_topology and L11_routing_order,
+// Builds it from L11_netPerm / L11_fromN / L11_toN (1-based, as produced by
+// L11_set_network_topology and L11_routing_order,
 // src/mRM/mo_mrm_net_startup.f90:630-886).  Fails (returns false, message in
 // err) unless netPerm is a permutation of the links in which every link comes
 // after all links that drain into its source node -- the order the reference
-// routes in (src/mRM/mo_mrm_routing.f90:435-459).
-bool build_level_network(int32_t n_nodes, int32_t n_outlets, const int32_t *net_perm, const int32_t *from_n,
-                         const int32_t *to_n, LevelNetwork &out, std::string &err);
+// routes in (src/mRM/mo_mrm_routing.f90:435-459).  `cap`: most nodes a block.
+bool build_route_network(int32_t n_nodes, int32_t n_outlets, const int32_t *net_perm, const int32_t *from_n,
+                         const int32_t *to_n, int32_t cap, RouteNetwork &out, std::string &err);
 
 // Routing order of L11_routing_order (src/mRM/mo_mrm_net_startup.f90:728-886)
 // computed with per-link counts of unranked upstream links instead of the

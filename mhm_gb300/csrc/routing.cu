@@ -1,20 +1,20 @@
-// routing.cu -- mRM L1->L11 runoff accumulation and Muskingum link routing,
-// time-chunked and level-synchronous.
+// routing.cu -- mRM L1->L11 runoff accumulation and Muskingum link routing.
 //
 // The reference advances every link one step at a time in netPerm order
 // (L11_routing, src/mRM/mo_mrm_routing.f90:380-481).  The per-link recurrence
 // only reads the link's own previous step and the same-step outflow of its
-// upstream links, so a whole chunk of steps of one link can run as soon as the
-// chunk of every upstream link is done: links are grouped into topological
-// levels and each level advances its links through the full chunk.  Inflow
-// sums at confluences keep the reference's order (upstream links in netPerm
-// rank order, then the node's own qOUT), so results are bit-identical.
-#include <atomic>
+// upstream links, so a chunk of steps runs through the river network as a
+// pipeline, each node one step behind the node upstream.  Inflow sums at
+// confluences keep the reference's order (upstream links in netPerm rank
+// order, then the node's own qOUT), so results are bit-identical.
 #include <cstdint>
+#include <type_traits>
 
 #include "bounds.cuh"
 #include "calendar.h"
+#include "fp64i.h"
 #include "mhm_kernels.cuh"
+#include "network.h"
 
 namespace mhm {
 
@@ -60,147 +60,252 @@ __global__ void __launch_bounds__(256) runoff_acc_kernel(const AccArgs a)
     a.qout[((size_t)m * a.n_steps + t) * L + pos] = q;
 }
 
-// One (member, node) of a wavefront tick: the node advances its sub-chunk
-// (tick - level) of `sub` <= SUB steps.  L11_routing body,
-// src/mRM/mo_mrm_routing.f90:435-478.  Inflow sums keep the reference order:
-// per step, ((0 + qTR(up_1)) + qTR(up_2) + ...) + qOUT, upstream links in
-// netPerm rank order; the upstream series of the whole sub-chunk are loaded
-// first (independent loads), then the Muskingum recurrence runs.  Everything
-// another thread wrote in an earlier tick (routed outflow, node states) is
-// read through L2 (ld.global.cg), so the function is also correct where
-// consecutive ticks run in one launch on different SMs.
-template <int SUB>
-__device__ __forceinline__ void route_item(const RouteArgs &a, const int m, const int pos, const int tick)
+// A step of an exported outflow series: the value and the number of the step,
+// counted on through all launches, in one 16-byte word that is read and
+// written whole.  A reader that finds the number it expects has the value; no
+// other ordering is needed, and a word left by an earlier launch never matches.
+__device__ __forceinline__ void put_step(longlong2 *p, double v, uint64_t id)
 {
-    // the item's own words first, all in flight together (every index is in
-    // range for any member and position; only the upstream reads depend on them)
+    asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(id)
+                 : "memory");
+}
+__device__ __forceinline__ void get_step(const longlong2 *p, uint64_t &v, uint64_t &id)
+{
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(v), "=l"(id)
+                 : "l"(p)
+                 : "memory");
+}
+
+// Reads a step until it is there.  The wait has a limit: when it runs out, or
+// another block's did, the launch is marked and false comes back.
+__device__ bool wait_step(const RouteArgs &a, const longlong2 *p, uint64_t id, uint64_t &v)
+{
+    uint64_t got = ~id;
+    for (int polls = 0; got != id; ++polls) {
+        volatile uint32_t *ab = a.abort;
+        if (polls > a.max_polls || ((polls & 63) == 63 && *ab == a.launch)) {
+            *ab = a.launch;
+            *reinterpret_cast<volatile int32_t *>(a.timed_out) = 1;
+            return false;
+        }
+        get_step(p, v, got);
+    }
+    return true;
+}
+
+// One block of the network for one member: a thread per node, a step per tick,
+// each node `lag` ticks behind the block's first.  L11_routing body,
+// src/mRM/mo_mrm_routing.f90:435-478: ((0 + qTR(up_1)) + qTR(up_2) + ...) +
+// qOUT, then the Muskingum recurrence.
+//
+// What bounds it: the tick, a chain of dependent FP64 operations (64 cycles
+// each on this GPU, three plus one per upstream link) and a block barrier; a
+// chunk of T steps takes T ticks plus the length of the river.  So everything a
+// tick reads is already on the chip: outflows pass from node to node through a
+// ring in shared memory, a node's own runoff and the outflows of other blocks
+// are fetched a round of S ticks ahead.  A block exports the outflow of its
+// pieces' last nodes to device memory, step by step.  Measured (one chunk of
+// 240 steps): 62,500 nodes, 1,478 deep, 2.1 ms; the same on a 1,458-deep grid
+// 2.2-2.4 ms; 576 nodes 0.20 ms.  A launch (or a cluster barrier) per wavefront
+// of all nodes, whose loads all came from device memory, took 16.1, 27.9 and
+// 0.69 ms.  64 nodes a block: with 32 a 576-node network takes 0.24 ms (more
+// hand-overs), with 128 the deep one gains nothing (the FP64 pipe of the SM is
+// shared by more warps a tick).  S = 8 covers a device-memory load; S = 4 hands
+// over sooner, 6-8 % faster where the river is longer than the chunk and as
+// much slower where it is not.
+//
+// Blocks take (network block, member) pairs from a counter, in an order in
+// which a pair waits only on pairs taken before it.  So whatever the number of
+// resident blocks, the oldest running one waits on nothing unfinished and the
+// launch ends; the limit in wait_step only guards against a defect.
+template <int S>
+__global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs a)
+{
+    // by tick: the outflows of the block's nodes, then of the series it takes,
+    // then a slot that stays +0 (the upstream link of a node without one)
+    constexpr int kSlots = 2 * kRouteBlock + 1, kZero = 2 * kRouteBlock;
+    __shared__ double ring[2 * S][kSlots];
+    __shared__ double own_q[2 * S][kRouteBlock]; // the nodes' own runoff by tick
+    __shared__ uint32_t s_pair;
+    const int tid = threadIdx.x;
+    if (tid == 0) s_pair = atomicAdd(a.ticket, 1u) - a.ticket0;
+    __syncthreads();
+    const int b = (int)(s_pair / (uint32_t)a.n_members), m = (int)(s_pair - (uint32_t)b * a.n_members);
+    if (a.member_step0 && a.member_step0[m] < 0) return; // idle member: routing states untouched
+    const int p0 = __ldg(a.blk_ptr + b), n = __ldg(a.blk_ptr + b + 1) - p0;
+    const int e0 = __ldg(a.ext_ptr + b), ne = __ldg(a.ext_ptr + b + 1) - e0;
+    const int nT = a.n_steps;
+    const int rounds = (nT + __ldg(a.blk_lag + b) + S - 1) / S;
     const int64_t L = a.n_nodes;
     const size_t ms = (size_t)m * L;
-    const int level = __ldg(a.pos_level + pos);
-    const int ub = __ldg(a.up_ptr + pos), ue = __ldg(a.up_ptr + pos + 1);
-    const int flags = __ldg(a.pos_flags + pos);
-    double qtin1 = __ldcg(a.qtin1 + ms + pos);
-    double qtr1 = __ldcg(a.qtr1 + ms + pos);
-    const double c1 = __ldg(a.C1 + ms + pos);
-    const double c2 = __ldg(a.C2 + ms + pos);
-    if (a.member_step0 && a.member_step0[m] < 0) return; // idle member: routing states untouched
-    const int s = tick - level;
-    const int t0 = s * a.sub;
-    if (s < 0 || t0 >= a.n_steps) return;
-    const int nt = min(a.sub, a.n_steps - t0);
-    const size_t base = ((size_t)m * a.n_steps + t0) * L; // row t0 of member m
-    const bool is_link = flags & 1;
-    const bool add_qout = flags & 2;
-    const bool cut = flags & 4; // mo_mrm_routing.f90:447-452
-    double qtin[SUB];
+    longlong2 *const qx = a.qx + (size_t)m * a.n_exports * a.qx_stride;
+
+    const bool own = tid < n;
+    const int pos = p0 + tid;
+    int lag = 0, flags = 0, ex = -1, nu = 0, hub = -1;
+    int up[kRouteUps]; // the upstream links' slots
 #pragma unroll
-    for (int t = 0; t < SUB; ++t) qtin[t] = 0.0; // netNode_qTIN(:, IT) = 0
-    for (int j = ub; j < ue; ++j) {
-        const int up_pos = __ldg(a.up_pos + j);
-        if (!bc_ok(BC_ROUTE_UP, up_pos, L)) continue;
-        const double *up = a.qtr + base + up_pos;
+    for (int j = 0; j < kRouteUps; ++j) up[j] = kZero;
+    double qtin1 = 0.0, qtr1 = 0.0, c1 = 0.0, c2 = 0.0;
+    if (own) {
+        lag = __ldg(a.pos_lag + pos);
+        flags = __ldg(a.pos_flags + pos);
+        ex = __ldg(a.pos_export + pos);
+        const int4 w = __ldg(reinterpret_cast<const int4 *>(a.pos_ups) + pos);
+        const int v[kRouteUps] = {(int16_t)w.x, w.x >> 16, (int16_t)w.y, w.y >> 16,
+                                  (int16_t)w.z, w.z >> 16, (int16_t)w.w, w.w >> 16};
+        if (v[0] == -2) {
+            hub = v[1] + (v[2] << 15);
+        } else {
 #pragma unroll
-        for (int t = 0; t < SUB; ++t)
-            if (t < nt) qtin[t] = qtin[t] + __ldcg(up + (size_t)t * L);
+            for (int j = 0; j < kRouteUps; ++j)
+                if (v[j] >= 0 && bc_ok(BC_ROUTE_UP, v[j], kZero)) {
+                    up[j] = v[j];
+                    nu = j + 1;
+                }
+        }
+        qtin1 = a.qtin1[ms + pos];
+        qtr1 = a.qtr1[ms + pos];
+        c1 = __ldg(a.C1 + ms + pos);
+        c2 = __ldg(a.C2 + ms + pos);
     }
-    if (add_qout && bc_ok(BC_ROUTE_QOUT, (t0 + nt - 1) / a.rdiv, a.n_qsteps)) {
-        const double *qo = a.qout + (size_t)m * a.n_qsteps * L + pos;
+    const bool is_link = flags & 1, add_qout = flags & 2, cut = flags & 4; // cut: mo_mrm_routing.f90:447-452
+    const bool keep_qmod = own && (a.qmod_all || (flags & 16));
+    const double *qo = a.qout + (size_t)m * a.n_qsteps * L + pos;
+    double *qm = a.qmod + (size_t)m * nT * L + pos;
+    longlong2 *const out = ex >= 0 ? qx + (size_t)ex * a.qx_stride : nullptr;
+    // warp-wide facts, so that a tick branches on them without divergence.
+    // Adding the +0 of a link a node does not have changes nothing (its sum is
+    // never -0), so all lanes of a warp add as many links as the longest list;
+    // likewise the +0 runoff of a node that adds none.
+    const int nu_warp = (int)__reduce_max_sync(~0u, (unsigned)nu);
+    const bool hub_warp = __any_sync(~0u, hub >= 0), cut_warp = __any_sync(~0u, cut);
+    const bool out_warp = __any_sync(~0u, ex >= 0), qmod_warp = __any_sync(~0u, keep_qmod);
+    const int lag_hi = (int)__reduce_max_sync(~0u, (unsigned)lag);
+    const int lag_lo = (int)__reduce_min_sync(~0u, own ? (unsigned)lag : 0xffffu);
+
+    // series tid of the block's list
+    const int x_in = tid < ne ? __ldg(a.ext_export + e0 + tid) : 0;
+    const bool take = tid < ne && bc_ok(BC_ROUTE_UP, x_in, a.n_exports);
+    const longlong2 *in = take ? qx + (size_t)x_in * a.qx_stride : nullptr;
+    const int in_lag = take ? __ldg(a.ext_lag + e0 + tid) : 0;
+    bool bad = false;
+    uint64_t xv[S], xi[S];
+
+    // what round r reads, S ticks from S * r
+    auto fetch = [&](int r) {
+        if (add_qout) {
+            const int t0 = r * S - lag, h0 = (r & 1) * S;
 #pragma unroll
-        for (int t = 0; t < SUB; ++t)
-            if (t < nt) qtin[t] = qtin[t] + __ldcg(qo + (size_t)((t0 + t) / a.rdiv) * L);
-    }
-#pragma unroll
-    for (int t = 0; t < SUB; ++t) {
-        if (t < nt) {
-            const size_t row = base + (size_t)t * L;
-            if (is_link) {
-                double qtr = qtr1 + c1 * (qtin1 - qtr1) + c2 * (qtin[t] - qtin1);
-                if (cut) qtr = 0.0;
-                a.qtr[row + pos] = qtr;
-                qtr1 = qtr;
+            for (int j = 0; j < S; ++j) {
+                const int t = t0 + j;
+                if ((unsigned)t < (unsigned)nT) {
+                    const int row = a.rdiv == 1 ? t : t / a.rdiv;
+                    if (!bc_ok(BC_ROUTE_QOUT, row, a.n_qsteps)) continue;
+                    const unsigned dst = (unsigned)__cvta_generic_to_shared(&own_q[h0 + j][tid]);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(qo + (size_t)row * L)
+                                 : "memory");
+                }
             }
-            qtin1 = qtin[t];
-            a.qmod[row + pos] = 0.0 + qtin[t]; // L11_qMod = (0 + Qmod) / real(rout_loop = 1)
         }
+        if (take) {
+            const int t0 = r * S - in_lag;
+#pragma unroll
+            for (int j = 0; j < S; ++j) {
+                xv[j] = xi[j] = 0;
+                if ((unsigned)(t0 + j) < (unsigned)nT) get_step(in + t0 + j, xv[j], xi[j]);
+            }
+        }
+    };
+    auto land = [&](int r) { // ... into shared memory: a tick reads the row of the tick before it
+        if (take) {
+            const int t0 = r * S - in_lag, h0 = (r & 1) * S;
+#pragma unroll
+            for (int j = 0; j < S; ++j) {
+                const uint64_t id = a.done0 + (uint64_t)(t0 + j);
+                if ((unsigned)(t0 + j) < (unsigned)nT && xi[j] != id && !bad)
+                    bad = !wait_step(a, in + t0 + j, id, xv[j]);
+                ring[(h0 + j - 1) & (2 * S - 1)][kRouteBlock + tid] = __longlong_as_double((long long)xv[j]);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    };
+    // one tick; `k` its number, `i` its row of the ring
+    auto tick = [&](int k, int i) {
+        const double *row = ring[(i - 1) & (2 * S - 1)];
+        const int t = k - lag;
+        const double qo_t = own_q[i][tid];
+        double q = row[up[0]];
+        if (nu_warp > 1) {
+            const double v1 = row[up[1]], v2 = row[up[2]];
+            q = q + v1;
+            if (nu_warp > 2) q = q + v2;
+            if (nu_warp > 3) {
+#pragma unroll
+                for (int u = 3; u < kRouteUps; ++u)
+                    if (u < nu_warp) q = q + row[up[u]];
+            }
+        }
+        if (hub_warp && hub >= 0) {
+            const int u1 = __ldg(a.hub_ptr + hub + 1);
+            for (int u = __ldg(a.hub_ptr + hub); u < u1; ++u) {
+                const int x = __ldg(a.hub_ups + u);
+                if (!bc_ok(BC_ROUTE_UP, x, a.n_exports)) continue;
+                uint64_t v = 0;
+                if (!bad) bad = !wait_step(a, qx + (size_t)x * a.qx_stride + t, a.done0 + (uint64_t)t, v);
+                q = q + __longlong_as_double((long long)v);
+            }
+        }
+        q = q + qo_t;
+        // 0 + (-0) is +0: the sum starts at netNode_qTIN(:, IT) = 0
+        q = hm_sel(hm_d2b(q) == 0x8000000000000000ULL, 0.0, q);
+        const double keep = qtr1 + c1 * (qtin1 - qtr1);
+        double qtr = keep + c2 * (q - qtin1);
+        if (cut_warp) qtr = hm_sel(cut, 0.0, qtr);
+        ring[i][tid] = qtr;
+        if (out_warp && out) put_step(out + t, qtr, a.done0 + (uint64_t)t);
+        qtr1 = qtr;
+        qtin1 = q;
+        if (qmod_warp && keep_qmod) qm[(size_t)t * L] = q; // L11_qMod = (0 + Qmod) / real(rout_loop = 1)
+    };
+    if (tid < 2 * S) ring[tid][kZero] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 2 * S; ++i) own_q[i][tid] = 0.0;
+    fetch(0);
+    land(0);
+    if (__syncthreads_or(bad)) return;
+
+    auto round = [&](int r, auto half) {
+        constexpr int h0 = decltype(half)::value * S;
+        if (r + 1 < rounds) fetch(r + 1);
+        if (r * S >= lag_hi && (r + 1) * S - lag_lo <= nT) { // every node of the warp has a step in every tick
+#pragma unroll
+            for (int j = 0; j < S; ++j) {
+                tick(r * S + j, h0 + j);
+                if (j + 1 < S) __syncthreads();
+            }
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < S; ++j) {
+                const int k = r * S + j;
+                if ((unsigned)(k - lag) < (unsigned)nT) tick(k, h0 + j);
+                if (j + 1 < S) __syncthreads();
+            }
+        }
+        if (r + 1 < rounds) land(r + 1);
+        return __syncthreads_or(bad) != 0;
+    };
+    for (int r = 0; r < rounds; r += 2) {
+        if (round(r, std::integral_constant<int, 0>())) return;
+        if (r + 1 < rounds && round(r + 1, std::integral_constant<int, 1>())) return;
     }
-    a.qtin1[ms + pos] = qtin1;
-    a.qtr1[ms + pos] = qtr1;
-}
-
-// One wavefront tick per launch: threads over (member, position) of the
-// levels the tick spans.
-template <int SUB>
-__global__ void __launch_bounds__(128) route_tick_kernel(const RouteArgs a)
-{
-    const int width = a.pos_end - a.pos_begin;
-    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (int64_t)width * a.n_members) return;
-    const int m = (int)(gid / width);
-    route_item<SUB>(a, m, a.pos_begin + (int)(gid - (int64_t)m * width), a.tick);
-}
-
-// All ticks of a chunk in one launch: each thread-block cluster walks the
-// wavefront of its members (m = cluster, cluster + clusters, ...), its CTAs
-// sharing the (member, position) items of a tick, with a hardware cluster
-// barrier between ticks.  The CTAs of a cluster are co-scheduled by the
-// hardware and every thread reaches every barrier (no thread leaves the tick
-// loop early), so no wait depends on work outside the cluster; clusters never
-// wait on one another.  The barrier's release/acquire orders a tick's stores
-// before the next tick's L2 reads.
-__device__ __forceinline__ unsigned cluster_sreg_rank()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_sreg_size()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_sreg_id()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_sreg_count()
-{
-    unsigned r;
-    asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_barrier()
-{
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// 512 threads per CTA: one item per thread in the ticks of a 62,500-node
-// network on a 16-CTA cluster (measured: 128 / 256 / 512 threads took 21.7 /
-// 17.6 / 16.2 ms for its 240-step chunk)
-constexpr int kWalkThreads = 512;
-
-template <int SUB>
-__global__ void __launch_bounds__(kWalkThreads) route_walk_kernel(const RouteArgs a, const RouteWalk w)
-{
-    const int cs = (int)cluster_sreg_size(), rank = (int)cluster_sreg_rank();
-    const int cid = (int)cluster_sreg_id(), ncl = (int)cluster_sreg_count();
-    // items interleaved over the CTAs (item i on CTA i % cs): a tick's work
-    // spreads over every SM of the cluster, whose FP64 pipes bound it
-    const int nthr = cs * (int)blockDim.x;
-    const int tid = (int)threadIdx.x * cs + rank;
-    const int mc = cid < a.n_members ? (a.n_members - cid + ncl - 1) / ncl : 0; // this cluster's members
-    for (int k = 0; k < w.n_ticks; ++k) {
-        const int lo = max(0, k - w.n_sub + 1), hi = min(k, w.n_levels - 1);
-        const int pb = __ldg(w.level_ptr + lo), pe = __ldg(w.level_ptr + hi + 1);
-        const int width = pe - pb;
-        const int items = width * mc; // < 2^31: positions x members of one context
-        for (int i = tid; i < items; i += nthr) {
-            const int mi = i / width;
-            route_item<SUB>(a, cid + mi * ncl, pb + (i - mi * width), k);
-        }
-        cluster_barrier();
+    if (own) {
+        a.qtin1[ms + pos] = qtin1;
+        if (is_link) a.qtr1[ms + pos] = qtr1;
+        if (a.qmod_last) a.qmod_last[ms + pos] = qtin1;
+        if (a.qout_last) a.qout_last[ms + pos] = __ldg(qo + (size_t)(a.n_qsteps - 1) * L);
     }
 }
 
@@ -361,72 +466,15 @@ cudaError_t launch_runoff_acc(const AccArgs &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_route_tick(const RouteArgs &a, cudaStream_t s)
+// `round`: steps fetched ahead at a time, 1..16
+cudaError_t launch_route_flow(const RouteArgs &a, int round, cudaStream_t s)
 {
-    const int64_t n = (int64_t)(a.pos_end - a.pos_begin) * a.n_members;
-    if (n == 0) return cudaSuccess;
-    const unsigned grid = (unsigned)((n + 127) / 128);
-    if (a.sub <= 4) route_tick_kernel<4><<<grid, 128, 0, s>>>(a);
-    else if (a.sub <= 8) route_tick_kernel<8><<<grid, 128, 0, s>>>(a);
-    else if (a.sub <= 16) route_tick_kernel<16><<<grid, 128, 0, s>>>(a);
+    if (a.n_members < 1 || a.n_steps < 1) return cudaSuccess;
+    const unsigned grid = (unsigned)(a.n_blocks * a.n_members);
+    if (round <= 4) route_flow_kernel<4><<<grid, kRouteBlock, 0, s>>>(a);
+    else if (round <= 16) route_flow_kernel<8><<<grid, kRouteBlock, 0, s>>>(a);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
-}
-
-// Clusters of `cs` CTAs (4, 8 or 16; 16 is a non-portable size, and a size
-// no SM group of the device can hold falls back to the next smaller one), at
-// most one per member and no more than can be resident at once.  The
-// occupancy answer is kept per (device, SUB, cluster size).
-template <int SUB>
-static cudaError_t launch_route_walk_t(const RouteArgs &a, const RouteWalk &w, int cs, cudaStream_t s)
-{
-    constexpr int kDevs = 16;
-    static std::atomic<int> max_active[kDevs][3] = {}; // 0: not queried yet; -1: does not fit
-    auto kern = route_walk_kernel<SUB>;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kWalkThreads, 1, 1);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    for (; cs >= 4; cs /= 2) {
-        const int ci = cs == 4 ? 0 : cs == 8 ? 1 : 2;
-        at[0].val.clusterDim.x = (unsigned)cs;
-        int mc = dev < kDevs ? max_active[dev][ci].load() : 0;
-        if (mc == 0) {
-            if (cs > 8) {
-                e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                if (e != cudaSuccess) return e;
-            }
-            cfg.gridDim = dim3((unsigned)cs, 1, 1);
-            e = cudaOccupancyMaxActiveClusters(&mc, kern, &cfg);
-            if (e != cudaSuccess) return e;
-            if (mc < 1) mc = -1;
-            if (dev < kDevs) max_active[dev][ci].store(mc);
-        }
-        if (mc < 1) continue;
-        const int ncl = a.n_members < mc ? a.n_members : mc;
-        cfg.gridDim = dim3((unsigned)(ncl * cs), 1, 1);
-        return cudaLaunchKernelEx(&cfg, kern, a, w);
-    }
-    return cudaErrorInvalidConfiguration;
-}
-
-cudaError_t launch_route_walk(const RouteArgs &a, const RouteWalk &w, int cs, cudaStream_t s)
-{
-    if (a.n_members < 1 || w.n_ticks < 1) return cudaSuccess;
-    if (cs != 4 && cs != 8 && cs != 16) return cudaErrorInvalidValue;
-    if (a.sub <= 4) return launch_route_walk_t<4>(a, w, cs, s);
-    if (a.sub <= 8) return launch_route_walk_t<8>(a, w, cs, s);
-    if (a.sub <= 16) return launch_route_walk_t<16>(a, w, cs, s);
-    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_qmod_step(const QmodStepArgs &a, cudaStream_t s)

@@ -388,8 +388,8 @@ class MhmGpu:
 
     def autotune(self, tt0: int, n_steps: int, route: bool = True) -> dict:
         """Pick the fastest cell-chain register variant and routing sub-chunk
-        by timing n_steps from tt0 (states restored afterwards), then, with
-        `route`, the routing launch mode (per-tick graph or cluster walk)."""
+        by timing n_steps from tt0 (states restored afterwards); with `route`
+        also autotune_route."""
         occ = C.c_int32()
         sub = C.c_int32()
         ms = np.zeros(9)
@@ -400,8 +400,8 @@ class MhmGpu:
         return out
 
     def autotune_route(self, tt0: int, n_steps: int) -> dict:
-        """mhm_autotune_route: route_cluster 0 (per-tick graph), 4, 8, 16 timed;
-        the fastest is kept."""
+        """mhm_autotune_route: route_cluster 0, 4, 8, 16 timed (all launch the
+        same kernel)."""
         cl = C.c_int32()
         ms = np.zeros(4)
         self._check(self.L.mhm_autotune_route(self.ctx, tt0, n_steps, C.byref(cl), _d(ms)), "mhm_autotune_route")
