@@ -12,10 +12,11 @@
  * infinities ordered); the *_ieee variants are also false for NaN operands.
  * Division: hm_div(a, b) == a / b for all inputs; normal/zero operands with a
  * normal result take the integer path (float reciprocal seed, two Newton
- * steps in 64-bit fixed point, exact remainder correction, RNE); everything
- * else (subnormal, infinite, NaN, zero divisor, out-of-range results) uses
- * the native division.  hm_div_r(a, b, hm_recip_of(b)) is the same division
- * with the divisor's reciprocal computed beforehand.
+ * steps in 64-bit fixed point, one product, and the exact remainder where that
+ * leaves the rounding open); everything else (subnormal, infinite, NaN, zero
+ * divisor, out-of-range results) uses the native division.
+ * hm_div_r(a, b, hm_recip_of(b)) is the same division with the divisor's
+ * reciprocal computed beforehand.
  */
 #ifndef MHM_FP64I_H
 #define MHM_FP64I_H
@@ -82,10 +83,11 @@ HM_FN uint32_t hm_f2b(float f)
 }
 
 /* 64-bit fixed-point reciprocal of a divisor mantissa Mb in (2^52, 2^53):
- * inv ~ 2^116 / Mb < 2^64 from a float seed (~24 bits) and two Newton steps
- * y' = y (2 - Mb y / 2^116), which approach from below.  Depends on the
- * divisor only, so a divisor that stays fixed over many divisions (a cell's
- * soil parameters over a chunk of steps) needs it once: hm_recip_of. */
+ * floor(2^116 / Mb) from a float seed (~24 bits), two Newton steps
+ * y' = y (2 - Mb y / 2^116), which approach from below and end less than 3
+ * short, and the remainder.  Depends on the divisor only, so a divisor that
+ * stays fixed over many divisions (a cell's soil parameters over a chunk of
+ * steps) needs it once: hm_recip_of. */
 HM_FN uint64_t hm_recip_mant(uint64_t Mb)
 {
     const float fy = hm_frcp((float)(uint32_t)(Mb >> 29)); /* in (2^-24, 2^-23] */
@@ -102,22 +104,28 @@ HM_FN uint64_t hm_recip_mant(uint64_t Mb)
         const int64_t err_s = (int64_t)((e_hi << 12) | (e_lo >> 52));
         inv = inv + (uint64_t)(hm_smulhi((int64_t)(inv >> 1), err_s) * 2);
     }
+    uint64_t rem = (uint64_t)0 - Mb * inv; /* 2^116 - Mb*inv, below 3 Mb */
+    for (int it = 0; it < 2; ++it)
+        if (rem >= Mb) {
+            rem -= Mb;
+            inv += 1;
+        }
     return inv;
 }
 
-/* The reciprocal hm_div_r wants for divisor b (0 when b takes another path:
- * zero, subnormal, infinite, NaN or a power of two). */
+/* The reciprocal hm_div_r wants for divisor b: 0 for one that is zero,
+ * subnormal, infinite or NaN, the largest number for a power of two. */
 HM_FN uint64_t hm_recip_of(double b)
 {
     const uint64_t ub = hm_d2b(b);
     const uint32_t ebf = (uint32_t)(ub >> 52) & 0x7ffu;
     const uint64_t Mb = (ub & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
-    if (ebf - 1u >= 0x7feu || Mb == 0x0010000000000000ULL) return 0;
-    return hm_recip_mant(Mb);
+    if (ebf - 1u >= 0x7feu) return 0;
+    return Mb == 0x0010000000000000ULL ? 0xffffffffffffffffULL : hm_recip_mant(Mb);
 }
 
-/* a / b, correctly rounded, given inv = hm_recip_of(b) */
-HM_FN_BIG double hm_div_r(double a, double b, uint64_t inv)
+/* The divisions hm_div_r leaves: native, or by the exact remainder. */
+HM_FN_BIG double hm_div_rest(double a, double b, uint64_t inv)
 {
     const uint64_t ua = hm_d2b(a), ub = hm_d2b(b);
     const uint32_t eaf = (uint32_t)(ua >> 52) & 0x7ffu, ebf = (uint32_t)(ub >> 52) & 0x7ffu;
@@ -135,35 +143,43 @@ HM_FN_BIG double hm_div_r(double a, double b, uint64_t inv)
     }
     if (e > 1023 || e < -1022)
         return a / b; /* overflow or subnormal result: native path */
-    uint64_t Q;
-    hm_i128 R;
-    if (Mb == 0x0010000000000000ULL) { /* b is a power of two: exact */
-        Q = Ma << 2;
-        R = 0;
-    } else {
-        /* Q ~ floor(Ma * 2^54 / Mb) in [2^54, 2^55) */
-        Q = (hm_umulhi(Ma, inv) << 2) | ((Ma * inv) >> 62);
-        /* exact remainder Ma*2^54 - Q*Mb; |R| < 2^57, so modulo 2^64 suffices */
-        int64_t r = (int64_t)((Ma << 54) - Q * Mb);
-        for (int c = 0; c < 3; ++c) {
-            if (r < 0) {
-                Q -= 1;
-                r += (int64_t)Mb;
-            } else if (r >= (int64_t)Mb) {
-                Q += 1;
-                r -= (int64_t)Mb;
-            }
+    /* Q <= Ma * 2^54 / Mb in [2^54, 2^55), at most 2 too small; the remainder
+     * Ma*2^54 - Q*Mb is below 2^57, so modulo 2^64 suffices */
+    uint64_t Q = (hm_umulhi(Ma, inv) << 2) | ((Ma * inv) >> 62);
+    uint64_t r = (Ma << 54) - Q * Mb;
+    for (int c = 0; c < 3; ++c)
+        if (r >= Mb) {
+            Q += 1;
+            r -= Mb;
         }
-        R = r;
-    }
     /* round Q (55 bits: 53 + guard + round) to nearest even */
     uint64_t m53 = Q >> 2;
     const uint32_t g = (uint32_t)(Q & 3u);
-    const int sticky = R != 0;
-    if (g > 2 || (g == 2 && (sticky || (m53 & 1))))
+    if (g > 2 || (g == 2 && (r != 0 || (m53 & 1))))
         m53++;
     /* m53 in [2^52, 2^53]; a carry to 2^53 moves into the exponent field */
     return hm_b2d(sign | (((uint64_t)(e + 1022) << 52) + m53));
+}
+
+/* a / b, correctly rounded, given inv = hm_recip_of(b).
+ * The quotient to 63 bits is one high product, less than 4 too small; a
+ * quotient of doubles is never halfway between two doubles, so only where the
+ * half lies within those 4 (one division in 512) its remainder decides. */
+HM_FN_BIG double hm_div_r(double a, double b, uint64_t inv)
+{
+    const uint64_t ua = hm_d2b(a);
+    const uint32_t ha = hm_hi(ua), hb = hm_hi(hm_d2b(b)), sign = (ha ^ hb) & 0x80000000u;
+    int e = (int)((ha >> 20) & 0x7ffu) - (int)((hb >> 20) & 0x7ffu);
+    uint64_t q = hm_umulhi(ua << 11 | 0x8000000000000000ULL, inv);
+    if (!(q >> 63)) {
+        q <<= 1;
+        e -= 1;
+    }
+    if (inv != 0 && ((ha >> 20) & 0x7ffu) - 1u < 0x7feu && (uint32_t)(e + 1022) < 2045u && (hm_lo(q) & 0x7fcu) != 0x3fcu)
+        return hm_round63(q, e, sign);
+    if (inv != 0 && hm_abs_bits(ua) == 0)
+        return hm_b2d((uint64_t)sign << 32); /* +-0 / normal */
+    return hm_div_rest(a, b, inv);
 }
 
 /* a / b, correctly rounded */

@@ -198,6 +198,70 @@ def fixed_point_tables(lt):
         assert v < (1 << 64)
         print("  0x%016xULL, \\" % v)
     print("}")
+    one_sided_tables()
+
+
+# added to k so that k * ln2 is a product of unsigned numbers; its multiple of
+# ln2 (the same rounded constant) is taken off the table's logarithms again
+K_BIAS = 1100
+
+
+def one_sided_tables():
+    """The main paths' reduction: x = 2^k z, z = M 2^-52 in [1, 2), 256
+    sub-intervals by the top 8 bits of the mantissa, invc = A 2^-11 >= 1/z at the
+    interval's lower end, so that R = M*A - 2^63 is z*invc - 1 in Q63 exactly and
+    never negative (below 2^-7.6): every product is one of unsigned numbers.
+    log: -log(invc) - K_BIAS ln2 in Q70 (96 bits).  pow: -log2(invc) in Q64."""
+    ln2 = mp.log(2)
+    ln2_q70 = q(ln2, 70)
+    rows = []
+    for j in range(256):
+        zlo, zhi = 1 + mp.mpf(j) / 256, 1 + mp.mpf(j + 1) / 256 - mp.mpf(2) ** -52
+        A = int(mp.ceil(2048 / zlo))
+        assert A * zlo >= 2048 and A * zhi / 2048 - 1 < mp.mpf(2) ** mp.mpf("-7.6"), j
+        lnc = q(-mp.log(mp.mpf(A) / 2048), 70) - K_BIAS * ln2_q70
+        l2c = q(-mp.log(mp.mpf(A) / 2048, 2), 64)
+        assert 0 <= l2c < 1 << 64
+        rows.append((A, lnc & ((1 << 96) - 1), l2c))
+    print("/* ---- main paths of log / exp / pow: unsigned fixed point ---- */")
+    print("#define HM_U_KBIAS %d" % K_BIAS)
+    print("#define HM_U_LN2_Q70_W2 0x%xu" % (ln2_q70 >> 64))
+    print("#define HM_U_LN2_Q70_W1 0x%08xu" % ((ln2_q70 >> 32) & 0xFFFFFFFF))
+    print("#define HM_U_LN2_Q70_W0 0x%08xu" % (ln2_q70 & 0xFFFFFFFF))
+    # ln2/128 in Q103, words of a 96-bit number
+    c = q(ln2 / 128, 103)
+    assert c < 1 << 96
+    print("#define HM_U_LN2N_W2 0x%08xu" % (c >> 64))
+    print("#define HM_U_LN2N_W1 0x%08xu" % ((c >> 32) & 0xFFFFFFFF))
+    print("#define HM_U_LN2N_W0 0x%08xu" % (c & 0xFFFFFFFF))
+    print("#define HM_U_INVLN2N_Q24 0x%08xu /* floor(128/ln2 * 2^24) */" % int(mp.floor(128 / ln2 * 2 ** 24)))
+    # log1p(r) = r (1 - r (1/2 - r (1/3 - r (1/4 - r (1/5 - r (1/6 - r (1/7 - r/8)))))))
+    for n in range(5, 9):
+        print("#define HM_U_LOG_C%d 0x%08xu /* 1/%d, Q34 */" % (n, min(q(mp.mpf(1) / n, 34), 0xFFFFFFFF), n))
+    for n in range(2, 5):
+        print("#define HM_U_LOG_C%d 0x%016xULL /* 1/%d, Q63 */" % (n, q(mp.mpf(1) / n, 63), n))
+    # log2(1+r): the same over ln2
+    for n in range(4, 9):
+        print("#define HM_U_LOG2_C%d 0x%08xu /* Q33 */" % (n, q(1 / (n * ln2), 33)))
+    for n in range(1, 4):
+        print("#define HM_U_LOG2_C%d 0x%016xULL /* Q63 */" % (n, q(1 / (n * ln2), 63)))
+    # expm1(r) = r (1 + r (1/2 + r (1/6 + ...))), 2^g - 1 = g (ln2 + g (ln2^2/2 + ...))
+    for n in range(4, 7):
+        print("#define HM_U_EXP_C%d 0x%08xu /* Q36 */" % (n, q(1 / mp.factorial(n), 36)))
+        print("#define HM_U_EXP2_C%d 0x%08xu /* Q38 */" % (n, q(ln2 ** n / mp.factorial(n), 38)))
+    for n in range(1, 4):
+        print("#define HM_U_EXP_C%d 0x%016xULL /* Q63 */" % (n, q(1 / mp.factorial(n), 63)))
+        print("#define HM_U_EXP2_C%d 0x%016xULL /* Q63 */" % (n, q(ln2 ** n / mp.factorial(n), 63)))
+    print("/* log: {A | -log(invc) - bias in Q70, bits 64..95 << 32, its bits 0..63} x 256 */")
+    print("#define HM_U_LOG_TABLE_INIT { \\")
+    for A, lnc, _ in rows:
+        print("  {0x%016xULL, 0x%016xULL}, \\" % (A | (lnc >> 64) << 32, lnc & ((1 << 64) - 1)))
+    print("}")
+    print("/* pow: {A, -log2(invc) in Q64} x 256 */")
+    print("#define HM_U_LOG2_TABLE_INIT { \\")
+    for A, _, l2c in rows:
+        print("  {0x%016xULL, 0x%016xULL}, \\" % (A, l2c))
+    print("}")
 
 
 if __name__ == "__main__":

@@ -250,8 +250,10 @@ HM_FN double hm_pow_t(double x, double y, const uint64_t *ltab, const uint64_t *
  * number (k*ln2 + logc exact to 2^-107, log1p of the exact reduced argument
  * with relative error < 2^-61), exp from a Q64 argument (Taylor expm1 in
  * Q64, 2^(j/128) in Q63), and one final round-to-nearest-even to double.
- * No FP64 instruction is used on the main paths.  Accuracy (tests/
- * test_hmath.py): < 0.51 ulp for log and exp, < 0.6 ulp for pow.
+ * No FP64 instruction is used.  The _i2 functions take every argument; the
+ * unsigned main paths below them take the usual ones in less than half the
+ * instructions.  Accuracy (tests/test_hmath.py): < 0.51 ulp for log and exp,
+ * < 0.6 ulp for pow.
  * ====================================================================== */
 typedef __int128 hm_i128;
 typedef unsigned __int128 hm_u128;
@@ -298,12 +300,6 @@ HM_FN int hm_clz64(uint64_t x) /* x != 0 */
 #endif
 }
 
-HM_FN int hm_clz128(hm_u128 x) /* x != 0 */
-{
-    uint64_t hi = (uint64_t)(x >> 64);
-    return hi ? hm_clz64(hi) : 64 + hm_clz64((uint64_t)x);
-}
-
 /* Round mant * 2^(e - 63) (mant in [2^63, 2^64), `sticky` = nonzero bits
  * below mant) to the nearest double, ties to even; gradual underflow and
  * overflow to infinity. */
@@ -336,176 +332,8 @@ HM_FN double hm_make_double(int neg, uint64_t mant, int e, int sticky)
     return hm_b2d(sign | bits);
 }
 
-/* log(x) for positive normal-or-subnormal finite x as a Q116 fixed-point
- * number; also returns log1p of the reduced argument as a floating value
- * (neg, mant, e) and whether x lies in the two intervals around 1 where
- * log(x) == log1p(r) (near1).  Caller handles zero / negative / inf / NaN. */
-HM_FN hm_i128 hm_log_fx(uint64_t u, int *near1, int *tneg, uint64_t *tmant, int *te)
-{
-    int64_t kadj = 0;
-    if ((u >> 52) == 0) {
-        /* subnormal u * 2^-1074: shift the leading 1 to bit 52, which reads
-         * as the normal number (u << lz) * 2^-1074 = x * 2^lz */
-        const int lz = hm_clz64(u) - 11;
-        u <<= lz;
-        kadj = -lz;
-    }
-    const uint64_t tmp = u - HM_LOG_OFF;
-    const int64_t k = ((int64_t)tmp >> 52) + kadj;
-    const uint32_t i = (uint32_t)(tmp >> (52 - HM_LOG_NBITS)) & (HM_LOG_N - 1);
-    const uint64_t iz = u - (tmp & 0xfff0000000000000ULL);
-    const uint64_t M = (iz & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
-    const uint64_t A = HM_FXLOG_TAB[3 * i];
-    const int64_t R = (int64_t)(M * A) - ((int64_t)1 << 61); /* r = z*invc - 1 = R * 2^-61, exact */
-    const hm_i128 logc = (hm_i128)(((hm_u128)HM_FXLOG_TAB[3 * i + 1] << 64) | HM_FXLOG_TAB[3 * i + 2]);
-    *near1 = (k == 0) && (logc == 0);
-    if (R == 0) {
-        *tmant = 0;
-        return (hm_i128)k * (hm_i128)(((hm_u128)HM_FX_LN2_Q116_HI << 64) | HM_FX_LN2_Q116_LO) + logc;
-    }
-    /* log1p(r) = r * (1 + r * q(r)), q in Q63, r in Q64 */
-    const int64_t rq = R * 8;
-    int64_t q = HM_FX_LOG_C7;
-    q = HM_FX_LOG_C6 + hm_smulhi(rq, q);
-    q = HM_FX_LOG_C5 + hm_smulhi(rq, q);
-    q = HM_FX_LOG_C4 + hm_smulhi(rq, q);
-    q = HM_FX_LOG_C3 + hm_smulhi(rq, q);
-    q = HM_FX_LOG_C2 + hm_smulhi(rq, q);
-    const int64_t rqq = hm_smulhi(rq, q);                        /* r*q(r), Q63 */
-    const uint64_t f = (uint64_t)(((int64_t)1 << 62) + (rqq >> 1)); /* 1 + r*q(r), Q62 */
-    const uint64_t aR = (uint64_t)(R < 0 ? -R : R);
-    const int lz = hm_clz64(aR);
-    uint64_t mant = hm_umulhi(aR << lz, f);
-    const int lz2 = hm_clz64(mant);
-    mant <<= lz2;
-    const int e = 4 - lz - lz2; /* |log1p(r)| = mant * 2^(e - 63) */
-    *tneg = R < 0;
-    *tmant = mant;
-    *te = e;
-    /* S = k*ln2 + logc + log1p(r) in Q116 */
-    const int sh = e + 53;
-    hm_i128 tau = sh >= 0 ? (hm_i128)((hm_u128)mant << sh) : (hm_i128)(mant >> (-sh < 64 ? -sh : 63));
-    if (R < 0)
-        tau = -tau;
-    return (hm_i128)k * (hm_i128)(((hm_u128)HM_FX_LN2_Q116_HI << 64) | HM_FX_LN2_Q116_LO) + logc + tau;
-}
-
-/* Q116 -> nearest double */
-HM_FN double hm_q116_to_double(hm_i128 S)
-{
-    if (S == 0)
-        return 0.0;
-    const int neg = S < 0;
-    const hm_u128 a = (hm_u128)(neg ? -S : S);
-    const int lz = hm_clz128(a);
-    const hm_u128 n = a << lz;
-    return hm_make_double(neg, (uint64_t)(n >> 64), 11 - lz, (uint64_t)n != 0);
-}
-
-HM_FN_BIG double hm_log_i(double x)
-{
-    const uint64_t u = hm_d2b(x);
-    const uint32_t top = (uint32_t)(u >> 32);
-    if (top >= 0x7ff00000u) { /* +inf, NaN, or negative (sign bit set) */
-        if (u == 0x7ff0000000000000ULL)
-            return x;
-        if (hm_abs_bits(u) == 0)
-            return -HUGE_VAL; /* -0 */
-        return hm_b2d(0x7ff8000000000000ULL);
-    }
-    if (u == 0)
-        return -HUGE_VAL;
-    int near1, tneg, te;
-    uint64_t tmant;
-    const hm_i128 S = hm_log_fx(u, &near1, &tneg, &tmant, &te);
-    if (near1)
-        return tmant ? hm_make_double(tneg, tmant, te, 0) : 0.0;
-    return hm_q116_to_double(S);
-}
-
-/* exp(X * 2^-64) for a signed Q64 argument */
-HM_FN_BIG double hm_exp_q64(hm_i128 X)
-{
-    if (X > ((hm_i128)710 << 64))
-        return HUGE_VAL;
-    if (X < -((hm_i128)746 << 64))
-        return 0.0;
-    const int64_t t = (int64_t)(X >> 12);                     /* Q52 */
-    const int64_t kq = hm_smulhi(t, (int64_t)HM_FX_INVLN2N_Q54); /* x*128/ln2 in Q42 */
-    const int64_t k = (kq + ((int64_t)1 << 41)) >> 42;
-    const hm_i128 ln2n = (hm_i128)(((hm_u128)HM_FX_LN2N_Q116_HI << 64) | HM_FX_LN2N_Q116_LO);
-    const int64_t r = (int64_t)(X - (((hm_i128)k * ln2n) >> 52)); /* Q64, |r| < 2^-7 */
-    int64_t q = HM_FX_EXP_C6;
-    q = HM_FX_EXP_C5 + hm_smulhi(r, q);
-    q = HM_FX_EXP_C4 + hm_smulhi(r, q);
-    q = HM_FX_EXP_C3 + hm_smulhi(r, q);
-    q = HM_FX_EXP_C2 + hm_smulhi(r, q);                       /* Q63 */
-    const int64_t r2 = hm_smulhi(r, r);                       /* Q64 */
-    const int64_t p = r + hm_smulhi(r2, q) * 2;               /* expm1(r), Q64 */
-    const uint64_t T = HM_FXEXP_TAB[(uint32_t)k & 127u];      /* 2^(j/128), Q63 */
-    const uint64_t tp = hm_umulhi(T, (uint64_t)(p < 0 ? -p : p));
-    uint64_t y = p < 0 ? T - tp : T + tp;                     /* Q63 */
-    int e = (int)(k >> 7);
-    if (!(y >> 63)) {
-        y <<= 1;
-        e -= 1;
-    }
-    return hm_make_double(0, y, e, 0);
-}
-
-HM_FN double hm_exp_i(double x)
-{
-    const uint64_t u = hm_d2b(x);
-    const uint64_t a = hm_abs_bits(u);
-    if (a >= 0x4087500000000000ULL) { /* |x| >= 746, inf or NaN */
-        if (a > 0x7ff0000000000000ULL)
-            return x;
-        return (u >> 63) ? 0.0 : HUGE_VAL;
-    }
-    const int e = (int)(a >> 52) - 1023;
-    const uint64_t M = (a & 0x000fffffffffffffULL) | (a >> 52 ? 0x0010000000000000ULL : 0);
-    hm_i128 X;
-    if (e + 12 >= 0)
-        X = (hm_i128)((hm_u128)M << (e + 12));
-    else
-        X = (hm_i128)(e + 12 > -64 ? (M >> (-(e + 12))) : 0);
-    return hm_exp_q64((u >> 63) ? -X : X);
-}
-
-/* x**y for x >= 0 (Fortran real**real): exp(y * log(x)) with log kept in
- * fixed point (no rounding of the intermediate). */
-HM_FN_BIG double hm_pow_i(double x, double y)
-{
-    const uint64_t u = hm_d2b(x);
-    const uint64_t uy = hm_d2b(y);
-    const uint64_t ay = hm_abs_bits(uy);
-    if (ay == 0 || u == 0x3ff0000000000000ULL)
-        return 1.0;
-    const int ey = (int)(ay >> 52) - 1023;
-    if (u - 1 >= 0x7fefffffffffffffULL || ey > 40) {
-        /* x zero, negative, inf or NaN, or |y| >= 2^41 (inf/NaN included):
-         * the exp(y * log(x)) definition in FP64 */
-        return hm_exp_t(y * hm_log_t(x, HM_LOG_TAB), HM_EXP_TAB);
-    }
-    int near1, tneg, te;
-    uint64_t tmant;
-    const hm_i128 S = hm_log_fx(u, &near1, &tneg, &tmant, &te) >> 52; /* Q64, |S| < 2^74 */
-    const uint64_t My = (ay & 0x000fffffffffffffULL) | (ay >> 52 ? 0x0010000000000000ULL : 0);
-    const int neg = (S < 0) != (int)(uy >> 63);
-    const hm_u128 aS = (hm_u128)(S < 0 ? -S : S);
-    /* aS * My < 2^74 * 2^53: fits in 127 bits */
-    const hm_u128 prod = ((hm_u128)((uint64_t)(aS >> 64) * My) << 64) +
-                         (((hm_u128)hm_umulhi((uint64_t)aS, My) << 64) | (uint64_t)((uint64_t)aS * My));
-    const int sh = 52 - ey; /* >= 12 */
-    const hm_i128 P = (hm_i128)(sh < 127 ? prod >> sh : 0);
-    return hm_exp_q64(neg ? -P : P);
-}
-
-/* ---- the same fixed-point algorithms on explicit 64-bit limbs ----
- * Identical integers (and results) as hm_log_i / hm_exp_i / hm_pow_i above,
- * with fewer instructions: products of a small integer by a 128-bit
- * constant as two 64-bit products, shifts of 64-bit values into 128 bits,
- * and differences known to be small taken modulo 2^64. */
+/* ---- every argument: 64-bit limbs of Q116 (the path of the arguments the
+ * unsigned main paths below leave out) ---- */
 
 /* (hi, lo) = k * (chi, clo) for |k| < 2^32, as a signed 128-bit value */
 HM_FN void hm_mulk128(int64_t k, uint64_t chi, uint64_t clo, int64_t *rhi, uint64_t *rlo)
@@ -528,7 +356,10 @@ HM_FN void hm_add128(int64_t *hi, uint64_t *lo, int64_t bhi, uint64_t blo)
     *lo = l;
 }
 
-/* log(x) in Q116 as (hi, lo) limbs; same contract as hm_log_fx */
+/* log(x) for positive normal-or-subnormal finite x as a Q116 fixed-point
+ * number (hi, lo); also returns log1p of the reduced argument as a floating
+ * value (neg, mant, e) and whether x lies in the two intervals around 1 where
+ * log(x) == log1p(r) (near1).  Caller handles zero / negative / inf / NaN. */
 HM_FN void hm_log_fx2(uint64_t u, int64_t *Shi, uint64_t *Slo, int *near1, int *tneg, uint64_t *tmant, int *te)
 {
     int64_t kadj = 0;
@@ -784,11 +615,245 @@ HM_FN_BIG double hm_log10_i2(double x)
     return hm_q116_to_double2((int64_t)rhi, rlo);
 }
 
+/* ---- main paths: unsigned fixed point ----
+ * The reduction is one-sided (gen_hmath_tables.py, one_sided_tables): the
+ * reduced argument is never negative, so every product is of unsigned numbers,
+ * and a step of a polynomial is only as wide as its weight in the result asks
+ * for: the high-order steps multiply 32-bit words, the low-order ones drop the
+ * product of the low words (hm_mulhi_a).  A signed 64-bit high product takes
+ * 8.1 SM cycles a warp and 56 cycles of latency on this GPU, an unsigned one
+ * 4.7 and 40, a 32-bit one 1.3 and 10.  Errors before the one rounding: log
+ * 2^-69 absolute (outside |x - 1| < 2^-7), exp and pow 2^-62 relative; against
+ * 45 digits they round as many or more of 100,000 arguments a range correctly
+ * as the _i2 functions.  With the division's one-product path they took the
+ * 1e6-cell chunk's cell chain from 57.4 to 50.7 ms (which left it to the FP64
+ * pipe), 256 members from 475 to 383 ms and a 36-cell season from 19.4 to
+ * 14.2 ms.  Arguments outside the ranges below take the _i2 functions. */
+#if defined(__CUDACC__)
+struct __attribute__((aligned(16))) hm_w2 {
+    uint64_t a, b;
+};
+#else
+struct hm_w2 {
+    uint64_t a, b;
+};
+#endif
+typedef struct hm_w2 hm_w2;
+static const hm_w2 hm_ulog_tab_h[256] = HM_U_LOG_TABLE_INIT;
+static const hm_w2 hm_ulog2_tab_h[256] = HM_U_LOG2_TABLE_INIT;
+#if defined(__CUDACC__)
+static __device__ const hm_w2 hm_ulog_tab_d[256] = HM_U_LOG_TABLE_INIT;
+static __device__ const hm_w2 hm_ulog2_tab_d[256] = HM_U_LOG2_TABLE_INIT;
+#endif
+#if defined(__CUDA_ARCH__)
+#define HM_ULOG_TAB hm_ulog_tab_d
+#define HM_ULOG2_TAB hm_ulog2_tab_d
+#else
+#define HM_ULOG_TAB hm_ulog_tab_h
+#define HM_ULOG2_TAB hm_ulog2_tab_h
+#endif
+
+HM_FN hm_w2 hm_ld2(const hm_w2 *p)
+{
+#if defined(__CUDA_ARCH__)
+    const ulonglong2 v = *(const ulonglong2 *)p;
+    hm_w2 r;
+    r.a = v.x;
+    r.b = v.y;
+    return r;
+#else
+    return *p;
+#endif
+}
+
+HM_FN uint32_t hm_umulhi32(uint32_t a, uint32_t b)
+{
+#if defined(__CUDA_ARCH__)
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+HM_FN uint32_t hm_hi(uint64_t a) { return (uint32_t)(a >> 32); }
+HM_FN uint32_t hm_lo(uint64_t a) { return (uint32_t)a; }
+HM_FN uint64_t hm_mulw(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+/* a * b / 2^64 from below, at most 3 too small (the product of the low words
+ * and two truncations) */
+HM_FN uint64_t hm_mulhi_a(uint64_t a, uint64_t b)
+{
+    return hm_mulw(hm_hi(a), hm_hi(b)) + hm_hi(hm_mulw(hm_hi(a), hm_lo(b))) + hm_hi(hm_mulw(hm_lo(a), hm_hi(b)));
+}
+
+/* y * 2^(e - 63), y in [2^63, 2^64), a normal result: to the nearest double */
+HM_FN double hm_round63(uint64_t y, int e, uint32_t sign)
+{
+    const uint64_t m = (y >> 11) + ((y >> 10) & 1); /* in [2^52, 2^53]: a carry moves into the exponent */
+    return hm_b2d(m + ((uint64_t)((uint32_t)(e + 1022) << 20 | sign) << 32));
+}
+
+/* log(x) for finite x >= 2^-1022 with |x - 1| >= 2^-7 */
+HM_FN double hm_log_u(uint64_t u)
+{
+    const uint32_t hi = hm_hi(u);
+    const hm_w2 t = hm_ld2(HM_ULOG_TAB + ((hi >> 12) & 255u));
+    const uint64_t M = (uint64_t)((hi & 0x000fffffu) | 0x00100000u) << 32 | hm_lo(u);
+    const uint64_t R = M * hm_lo(t.a) - 0x8000000000000000ULL; /* r in Q63, r < 2^-7.6 */
+    const uint64_t r64 = R << 1, r71 = R << 8;
+    const uint32_t r32 = hm_hi(r64), r39 = hm_hi(r71);
+    uint32_t v = HM_U_LOG_C7 - hm_umulhi32(r32, HM_U_LOG_C8); /* Q34 */
+    v = HM_U_LOG_C6 - hm_umulhi32(r32, v);
+    v = HM_U_LOG_C5 - hm_umulhi32(r32, v);
+    uint64_t w = HM_U_LOG_C4 - (hm_mulw(r39, v) >> 10); /* Q63 */
+    w = HM_U_LOG_C3 - hm_mulhi_a(r64, w);
+    w = HM_U_LOG_C2 - hm_mulhi_a(r64, w);
+    w = 0x8000000000000000ULL - hm_mulhi_a(r64, w);
+    const uint64_t P = hm_umulhi(r71, w); /* log1p(r), Q70 */
+    /* S = k ln2 - log(invc) + log1p(r), Q70, 96 bits */
+    const uint32_t kb = (hi >> 20) - 1023u + HM_U_KBIAS;
+    const uint64_t s0 = hm_mulw(kb, HM_U_LN2_Q70_W0);
+    const uint64_t s1 = hm_mulw(kb, HM_U_LN2_Q70_W1) + hm_hi(s0);
+    uint32_t sh = kb * HM_U_LN2_Q70_W2 + hm_hi(s1) + hm_hi(t.a);
+    uint64_t sl = (s1 << 32 | hm_lo(s0)) + t.b;
+    sh += sl < t.b;
+    sl += P;
+    sh += sl < P;
+    const uint32_t sign = sh & 0x80000000u;
+    if (sign) {
+        sl = (uint64_t)0 - sl;
+        sh = ~sh + (sl == 0);
+    }
+    /* the leading bit is one of 62 .. 80 */
+    uint32_t a = sh, b = hm_hi(sl), c = hm_lo(sl);
+    int e = 25; /* exponent of bit 95 */
+    if (a == 0) {
+        a = b;
+        b = c;
+        c = 0;
+        e = -7;
+    }
+#if defined(__CUDA_ARCH__)
+    const int lz = __clz((int)a);
+    a = __funnelshift_l(b, a, lz);
+    b = __funnelshift_l(c, b, lz);
+#else
+    const int lz = __builtin_clz(a);
+    if (lz) {
+        a = a << lz | b >> (32 - lz);
+        b = b << lz | c >> (32 - lz);
+    }
+#endif
+    return hm_round63((uint64_t)a << 32 | b, e - lz, sign);
+}
+
+/* 2^(j/128) (1 + p) in Q63 for p in Q70 */
+HM_FN uint64_t hm_exp_scale(uint32_t j, uint64_t p)
+{
+    const uint64_t T = HM_FXEXP_TAB[j];
+    return T + (hm_mulhi_a(T, p) >> 6);
+}
+
+/* exp(x) for 2^-8 <= |x| < 708 */
+HM_FN double hm_exp_u(uint64_t u)
+{
+    const uint32_t hi = hm_hi(u);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023; /* -8 .. 9 */
+    const uint32_t mh = (hi & 0x000fffffu) | 0x00100000u;
+    const uint64_t X = ((uint64_t)mh << 32 | hm_lo(u)) << (e + 19); /* |x| in Q71, modulo 2^64 */
+    const uint32_t m32 = mh << 11 | hm_lo(u) >> 21;                 /* |x| 2^(31 - e) */
+    const uint32_t v = hm_umulhi32(m32, HM_U_INVLN2N_Q24);          /* |x| 128/ln2 2^(23 - e), from below */
+    /* x = k ln2/128 + r with r in [0, ln2/128 (1 + 2^-8)): for x < 0 the
+     * multiple is rounded up, with a margin for v's error */
+    const int neg = hi >> 31;
+    const uint32_t k = neg ? ((v + 8u) >> (23 - e)) + 1u : v >> (23 - e);
+    const uint64_t kc = hm_mulw(k, HM_U_LN2N_W1) + hm_hi(hm_mulw(k, HM_U_LN2N_W0));
+    const uint64_t K = kc + ((uint64_t)(k * HM_U_LN2N_W2) << 32); /* k ln2/128 in Q71, modulo 2^64 */
+    const uint64_t r71 = neg ? K - X : X - K, r64 = r71 >> 7;
+    const uint32_t r32 = hm_hi(r64), r39 = hm_hi(r71);
+    uint32_t c = HM_U_EXP_C5 + hm_umulhi32(r32, HM_U_EXP_C6); /* Q36 */
+    c = HM_U_EXP_C4 + hm_umulhi32(r32, c);
+    uint64_t w = HM_U_EXP_C3 + (hm_mulw(r39, c) >> 12); /* Q63 */
+    w = HM_U_EXP_C2 + hm_mulhi_a(r64, w);
+    w = HM_U_EXP_C1 + hm_mulhi_a(r64, w);
+    const int32_t ks = neg ? -(int32_t)k : (int32_t)k;
+    uint64_t y = hm_exp_scale((uint32_t)ks & 127u, hm_mulhi_a(r71, w));
+    int n = ks >> 7;
+    if (!(y >> 63)) { /* r above ln2/128 and j = 127: past 2, the carry is lost */
+        y = y >> 1 | 0x8000000000000000ULL;
+        n += 1;
+    }
+    return hm_round63(y, n, 0);
+}
+
+/* x ** y for finite x >= 2^-1022, 2^-10 <= y < 2 and a normal result: 2 to the
+ * power of y (k + log2(z)); *ok says whether the result is normal */
+HM_FN double hm_pow_u(uint64_t u, uint64_t uy, int *ok)
+{
+    const uint32_t hi = hm_hi(u);
+    const hm_w2 t = hm_ld2(HM_ULOG2_TAB + ((hi >> 12) & 255u));
+    const uint64_t M = (uint64_t)((hi & 0x000fffffu) | 0x00100000u) << 32 | hm_lo(u);
+    const uint64_t R = M * hm_lo(t.a) - 0x8000000000000000ULL;
+    const uint64_t r64 = R << 1, r71 = R << 8;
+    const uint32_t r32 = hm_hi(r64), r39 = hm_hi(r71);
+    uint32_t v = HM_U_LOG2_C7 - hm_umulhi32(r32, HM_U_LOG2_C8); /* Q33 */
+    v = HM_U_LOG2_C6 - hm_umulhi32(r32, v);
+    v = HM_U_LOG2_C5 - hm_umulhi32(r32, v);
+    v = HM_U_LOG2_C4 - hm_umulhi32(r32, v);
+    uint64_t w = HM_U_LOG2_C3 - (hm_mulw(r39, v) >> 9); /* Q63 */
+    w = HM_U_LOG2_C2 - hm_mulhi_a(r64, w);
+    w = HM_U_LOG2_C1 - hm_mulhi_a(r64, w);
+    const uint64_t F = t.b + (hm_mulhi_a(r71, w) >> 6); /* log2(z), Q64 */
+    /* y in Q63, y F from its exact product, y k in 96 bits */
+    const uint32_t yh = hm_hi(uy);
+    const uint64_t Y = ((uint64_t)((yh & 0x000fffffu) | 0x00100000u) << 32 | hm_lo(uy))
+                       << ((int)(yh >> 20) - 1023 + 11);
+    const int32_t k = (int32_t)(hi >> 20) - 1023;
+    const uint64_t t0 = hm_mulw(hm_lo(Y), (uint32_t)k);
+    uint64_t t1 = hm_mulw(hm_hi(Y), (uint32_t)k) + hm_hi(t0);
+    if (k < 0) t1 -= Y;
+    const uint64_t yF = hm_umulhi(Y, F), yk = t1 << 32 | hm_lo(t0), T = yk + yF; /* Q63 */
+    const int32_t th = (int32_t)hm_hi(t1) + (T < yF);
+    const int32_t n = (int32_t)((uint32_t)th << 1 | hm_hi(T) >> 31);
+    const uint64_t g71 = T << 8, g64 = (T << 1) & 0x01ffffffffffffffULL;
+    const uint32_t g32 = hm_hi(g64), g39 = hm_hi(g71);
+    uint32_t c = HM_U_EXP2_C5 + hm_umulhi32(g32, HM_U_EXP2_C6); /* Q38 */
+    c = HM_U_EXP2_C4 + hm_umulhi32(g32, c);
+    w = HM_U_EXP2_C3 + (hm_mulw(g39, c) >> 14); /* Q63 */
+    w = HM_U_EXP2_C2 + hm_mulhi_a(g64, w);
+    w = HM_U_EXP2_C1 + hm_mulhi_a(g64, w);
+    *ok = (uint32_t)(n + 1022) < 2045u;
+    return hm_round63(hm_exp_scale((hm_hi(T) >> 24) & 127u, hm_mulhi_a(g71, w)), n, 0);
+}
+
 #ifndef HM_FP64_MATH
 HM_FN double hm_log10(double x) { return hm_log10_i2(x); }
-HM_FN double hm_log(double x) { return hm_log_i2(x); }
-HM_FN double hm_exp(double x) { return hm_exp_i2(x); }
-HM_FN double hm_pow(double x, double y) { return hm_pow_i2(x, y); }
+HM_FN_BIG double hm_log(double x)
+{
+    const uint64_t u = hm_d2b(x);
+    const uint32_t hi = hm_hi(u);
+    /* zero, subnormal, negative, inf, NaN, or |x - 1| < 2^-7 */
+    if (hi - 0x00100000u >= 0x7fe00000u || hi - 0x3fefc000u < 0x00006000u)
+        return hm_log_i2(x);
+    return hm_log_u(u);
+}
+HM_FN_BIG double hm_exp(double x)
+{
+    const uint64_t u = hm_d2b(x);
+    if (((hm_hi(u) & 0x7fffffffu) - 0x3f700000u) >= 0x40862000u - 0x3f700000u)
+        return hm_exp_i2(x);
+    return hm_exp_u(u);
+}
+HM_FN_BIG double hm_pow(double x, double y)
+{
+    const uint64_t u = hm_d2b(x), uy = hm_d2b(y);
+    if (hm_hi(u) - 0x00100000u < 0x7fe00000u && hm_hi(uy) - 0x3f500000u < 0x40000000u - 0x3f500000u) {
+        int ok;
+        const double r = hm_pow_u(u, uy, &ok);
+        if (ok)
+            return r;
+    }
+    return hm_pow_i2(x, y);
+}
 #else
 HM_FN double hm_log(double x) { return hm_log_t(x, HM_LOG_TAB); }
 HM_FN double hm_exp(double x) { return hm_exp_t(x, HM_EXP_TAB); }
