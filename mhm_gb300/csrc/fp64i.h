@@ -115,7 +115,7 @@ HM_FN uint64_t hm_recip_mant(uint64_t Mb)
 
 /* The reciprocal hm_div_r wants for divisor b: 0 for one that is zero,
  * subnormal, infinite or NaN, the largest number for a power of two. */
-HM_FN uint64_t hm_recip_of(double b)
+HM_FN_BIG uint64_t hm_recip_of(double b)
 {
     const uint64_t ub = hm_d2b(b);
     const uint32_t ebf = (uint32_t)(ub >> 52) & 0x7ffu;
@@ -175,14 +175,84 @@ HM_FN_BIG double hm_div_r(double a, double b, uint64_t inv)
         q <<= 1;
         e -= 1;
     }
-    if (inv != 0 && ((ha >> 20) & 0x7ffu) - 1u < 0x7feu && (uint32_t)(e + 1022) < 2045u && (hm_lo(q) & 0x7fcu) != 0x3fcu)
-        return hm_round63(q, e, sign);
-    if (inv != 0 && hm_abs_bits(ua) == 0)
-        return hm_b2d((uint64_t)sign << 32); /* +-0 / normal */
-    return hm_div_rest(a, b, inv);
+    if (hm_unlikely(inv == 0 || ((ha >> 20) & 0x7ffu) - 1u >= 0x7feu || (uint32_t)(e + 1022) >= 2045u ||
+                    (hm_lo(q) & 0x7fcu) == 0x3fcu)) {
+        if (inv != 0 && hm_abs_bits(ua) == 0)
+            return hm_b2d((uint64_t)sign << 32); /* +-0 / normal */
+        return hm_div_rest(a, b, inv);
+    }
+    return hm_round63(q, e, sign);
 }
 
 /* a / b, correctly rounded */
 HM_FN_BIG double hm_div(double a, double b) { return hm_div_r(a, b, hm_recip_of(b)); }
+
+/* ---- a horizon's uptake in one go ----
+ * With S the soil moisture, pw the wilting point, f the root fraction, a the
+ * remaining demand and den = FC - pw (inv = hm_recip_of(den), eden its biased
+ * exponent), the actual evapotranspiration of the Feddes stress
+ *     r = a * f                        (wet: S >= FC)
+ *     r = a * ((f * (S - pw)) / den)   (pw < S < FC)
+ * and the storage left, S - r, each of the five operations rounded to nearest
+ * even as in FP64, on the integer pipe: one unpacking and one packing instead
+ * of a trip to the FP64 pipe for each (64 cycles of it a warp).
+ * Returns 0, with nothing written, where the operands leave what it assumes:
+ * hm_uptake_par / hm_uptake_var in range, S and pw within 2^11 of each other,
+ * r below S / 2, and no carry or tie that needs more than 64 bits. */
+HM_FN uint64_t hm_top(uint64_t x) { return x << 11 | 0x8000000000000000ULL; } /* mantissa, leading bit at 63 */
+/* a 64-bit mantissa to 53 bits, ties to even (0 with the carry lost) */
+HM_FN uint64_t hm_rne11(uint64_t x) { return (x + 0x3ffu + ((hm_lo(x) >> 11) & 1u)) & 0xfffffffffffff800ULL; }
+/* positive, within 2^-200 .. 2^200 */
+HM_FN int hm_uptake_var(double x) { return hm_hi(hm_d2b(x)) - 0x33700000u < 0x19000000u; }
+/* the product of two mantissas, leading bit at 63, its low bits as a sticky
+ * bit; *e the exponent it adds */
+HM_FN uint64_t hm_mul_top(uint64_t a, uint64_t b, int *e)
+{
+    uint64_t h = hm_umulhi(a, b), l = a * b;
+    *e = 1;
+    if (!(h >> 63)) {
+        h = h << 1 | l >> 63;
+        l <<= 1;
+        *e = 0;
+    }
+    return h | (l != 0);
+}
+HM_FN int hm_uptake(double S_, double pw_, double f_, double a_, int wet, uint64_t inv, int eden, double *r_, double *left_)
+{
+    const uint64_t Sb = hm_d2b(S_), pb = hm_d2b(pw_), fb = hm_d2b(f_), ab = hm_d2b(a_);
+    const uint64_t S = hm_top(Sb);
+    const int es = (int)(hm_hi(Sb) >> 20);
+    uint64_t T = hm_top(fb); /* the stress factor */
+    int et = (int)(hm_hi(fb) >> 20), e;
+    if (!wet) {
+        const int d = es - (int)(hm_hi(pb) >> 20);
+        uint64_t D = S - (hm_top(pb) >> (d & 63)); /* exact */
+        const int lz = hm_clz64(D | 1);
+        D = hm_rne11(D << lz);
+        const uint64_t P = hm_rne11(hm_mul_top(D, T, &e));
+        uint64_t q = hm_umulhi(P, inv);
+        et += es - lz + e - eden;
+        if (!(q >> 63)) {
+            q <<= 1;
+            et -= 1;
+        }
+        T = (q + 0x400u) & 0xfffffffffffff800ULL;
+        if (d > 11 || (int32_t)(hm_hi(D) & hm_hi(P) & hm_hi(T)) >= 0 || (hm_lo(q) & 0x7fcu) == 0x3fcu)
+            return 0;
+    }
+    const uint64_t R = hm_rne11(hm_mul_top(hm_top(ab), T, &e));
+    const int er = (int)(hm_hi(ab) >> 20) + et + e - 1023;
+    const int d = es - er;
+    if ((uint32_t)(d - 2) > 60u || (int32_t)hm_hi(R) >= 0)
+        return 0;
+    const uint64_t y = R >> d, part = (y << d) != R;
+    uint64_t D = S - y - part;
+    const uint32_t up = (uint32_t)(hm_hi(D) >> 31) ^ 1u; /* below half the binade */
+    D = D << up | part;
+    const uint64_t m = (D >> 11) + ((hm_lo(D) & 0x7ffu) + ((hm_lo(D) >> 11) & 1u) > 0x400u);
+    *left_ = hm_b2d(m + ((uint64_t)(uint32_t)(es - (int)up - 1) << 52));
+    *r_ = hm_b2d((R >> 11) + ((uint64_t)(uint32_t)(er - 1) << 52));
+    return 1;
+}
 
 #endif /* MHM_FP64I_H */

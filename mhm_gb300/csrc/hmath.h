@@ -51,6 +51,9 @@
 
 #define HM_LOG_N (1 << HM_LOG_NBITS)
 
+/* a branch whose instructions go out of the way of the others' */
+#define hm_unlikely(c) __builtin_expect(!!(c), 0)
+
 HM_FN double hm_b2d(uint64_t b)
 {
 #if defined(__CUDA_ARCH__)
@@ -832,14 +835,14 @@ HM_FN_BIG double hm_log(double x)
     const uint64_t u = hm_d2b(x);
     const uint32_t hi = hm_hi(u);
     /* zero, subnormal, negative, inf, NaN, or |x - 1| < 2^-7 */
-    if (hi - 0x00100000u >= 0x7fe00000u || hi - 0x3fefc000u < 0x00006000u)
+    if (hm_unlikely(hi - 0x00100000u >= 0x7fe00000u || hi - 0x3fefc000u < 0x00006000u))
         return hm_log_i2(x);
     return hm_log_u(u);
 }
 HM_FN_BIG double hm_exp(double x)
 {
     const uint64_t u = hm_d2b(x);
-    if (((hm_hi(u) & 0x7fffffffu) - 0x3f700000u) >= 0x40862000u - 0x3f700000u)
+    if (hm_unlikely(((hm_hi(u) & 0x7fffffffu) - 0x3f700000u) >= 0x40862000u - 0x3f700000u))
         return hm_exp_i2(x);
     return hm_exp_u(u);
 }
