@@ -25,7 +25,7 @@ LIB = BUILD / "libmhm_gpu.so"
 # data-derived access, failures reported through a device status word
 LIB_BC = BUILD / "libmhm_gpu_bc.so"
 
-SOURCES = ["cell_chain.cu", "cell_chain_o6.cu", "cell_chain_o8.cu", "routing.cu", "probes.cu", "mpr.cu", "engine.cu",
+SOURCES = ["cell_chain.cu", "cell_chain_o6.cu", "cell_chain_o8.cu", "cell_chain_small.cu", "routing.cu", "probes.cu", "mpr.cu", "engine.cu",
            "network.cpp", "netbuild.cpp", "mpr_host.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -1,12 +1,15 @@
 // cell_chain.cu -- launchers of the cell-chain kernel (register variant for
 // 4 resident blocks per SM) and of the step-calendar kernel.  Variants sized
-// for 6 and 8 resident blocks per SM live in cell_chain_o6.cu / _o8.cu.
+// for 6 and 8 resident blocks per SM live in cell_chain_o6.cu / _o8.cu, the
+// kernel of small launches in cell_chain_small.cu.
 #include "cell_chain_impl.cuh"
 
 namespace mhm {
 
 cudaError_t launch_cell_chain_o6(const CellArgs &a, int H, cudaStream_t s);
 cudaError_t launch_cell_chain_o8(const CellArgs &a, int H, cudaStream_t s);
+bool cell_chain_fits_small(const CellArgs &a);
+cudaError_t launch_cell_chain_small(const CellArgs &a, cudaStream_t s);
 
 // Calendar of steps tt0 .. tt0+n-1: forcing row, month, day flags, day of year.
 __global__ void steps_fill_kernel(StepInfo *steps, int64_t tt0, int32_t n, int32_t jul_start, int32_t timestep,
@@ -71,6 +74,7 @@ cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
     if (H < 1 || H > kMaxHorizons) return cudaErrorInvalidValue;
     // per-step fluxes or aggregated outputs: one variant
     if (a.flux_aet || a.out.n_planes > 0) return launch_cell_chain_variant<4, true>(a, H, s);
+    if (cell_chain_fits_small(a)) return launch_cell_chain_small(a, s);
     switch (occ) {
     case 6: return launch_cell_chain_o6(a, H, s);
     case 8: return launch_cell_chain_o8(a, H, s);

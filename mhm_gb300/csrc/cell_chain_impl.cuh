@@ -133,32 +133,41 @@ __device__ __forceinline__ bool sm_frac_bounded(double sms, double beta)
     return hm_abs_bits(hm_d2b(sms)) < 0x7ff0000000000000ULL && hm_d2b(beta) - 1 < 0x7fefffffffffffffULL;
 }
 
-// The uptake of one horizon for the operands hm_uptake leaves: the actual
-// evapotranspiration and the storage left, in FP64.  mo_soil_moisture.f90:
-// 254-286 with the Feddes (:340-365) or Jarvis (:415-450) stress.  Out of line:
-// a block takes it for few lanes, and its instructions stay out of the loop.
-struct Uptake {
-    double aet, smh;
-};
-__device__ __noinline__ Uptake uptake_general(bool feddes, double aet, double smh, double sms, double fc, double pw,
-                                              double froots, uint64_t r_den, double jarvis, uint64_t r_jarvis)
+// The stress factor of one horizon, mo_soil_moisture.f90:340-365 (Feddes) and
+// :415-450 (Jarvis); den = FC - PW or SMs - PW.
+__device__ __forceinline__ double stress_factor(bool feddes, double smh, double fc, double pw, double froots,
+                                                double den, uint64_t r_den, double jarvis, uint64_t r_jarvis)
 {
     double stress;
     if (feddes) {
         const bool wet = hm_ge(smh, fc);
         stress = hm_sel(wet, froots, 0.0);
         // mo_soil_moisture.f90:358
-        if (!wet && hm_gt(smh, pw)) stress = hm_div_r(froots * (smh - pw), fc - pw, r_den);
+        if (!wet && hm_gt(smh, pw)) stress = hm_div_r(froots * (smh - pw), den, r_den);
     } else {
         // with SMs == PW the quotient can be NaN (0 / 0): IEEE
         // comparisons then leave the stress at 0 as the oracle does
-        double th = hm_div_r(smh - pw, sms - pw, r_den);
+        double th = hm_div_r(smh - pw, den, r_den);
         th = hm_sel(hm_lt_ieee(th, 0.0), 0.0, th);
         th = hm_sel(hm_gt_ieee(th, 1.0), 1.0, th);
         const bool wet = hm_ge_ieee(th, jarvis);
         stress = hm_sel(wet, froots, 0.0);
         if (!wet && hm_lt_ieee(th, jarvis)) stress = froots * hm_div_r(th, jarvis, r_jarvis);
     }
+    return stress;
+}
+
+// The uptake of one horizon for the operands hm_uptake leaves: the actual
+// evapotranspiration and the storage left, in FP64 (mo_soil_moisture.f90:
+// 254-286).  Out of line: a block takes it for few lanes, and its instructions
+// stay out of the loop.
+struct Uptake {
+    double aet, smh;
+};
+__device__ __noinline__ Uptake uptake_general(bool feddes, double aet, double smh, double sms, double fc, double pw,
+                                              double froots, uint64_t r_den, double jarvis, uint64_t r_jarvis)
+{
+    const double stress = stress_factor(feddes, smh, fc, pw, froots, feddes ? fc - pw : sms - pw, r_den, jarvis, r_jarvis);
     aet = aet * stress;
     aet = hm_sel(hm_lt0(aet), 0.0, aet);
     // enough: storage smh - aet, aet kept; else aet = smh - eps and
@@ -173,19 +182,24 @@ __device__ __noinline__ Uptake uptake_general(bool feddes, double aet, double sm
 }
 
 // The part of a cell's step above the soil -- meteo, canopy, snow and the sealed
-// bucket -- which depends on the forcing and on its own states only.
-template <bool LEAN> struct Surface {
+// bucket -- which depends on the forcing and on its own states only.  KEEP keeps
+// the meteo of a daily forcing row from hour to hour (it changes with the row,
+// the month and day or night) at the price of registers.
+template <bool LEAN, bool KEEP = false> struct Surface {
     // states
     double interc, snow, seal;
     // parameters (and parameter-only derived values)
     double ddinc, ddmax_s, ddnopre_s, dd_thr, tthresh, sthresh, fasp, harsam, lat_rad;
-    uint64_t r_sthresh; // reciprocal of a chunk-fixed divisor
+    uint64_t r_sthresh, r_nd; // reciprocals of chunk-fixed divisors
     bool sealed, sthresh_pos, dd_thr_ok;
     // of the month and LAI entry, and of the day
     int cur_key = -1, cur_doy = -1;
     double imax = 0.0, petlai = 0.0, petsurf = 0.0, evap = 0.0, rad = 0.0;
     uint64_t r_imax = 0, r_evap = 0;
+    size_t cur_f = ~(size_t)0;
+    int cur_day = -1;
     // of the step
+    double temp, prec;
     double pet, aet_can, prec_effect, melt, runoff_sealed, aet_sealed_act;
 
     __device__ __forceinline__ void load(const CellArgs &a, const double *P, const double *S, double fsealed, int k)
@@ -203,6 +217,7 @@ template <bool LEAN> struct Surface {
         harsam = par(P_HARSAM);
         lat_rad = (a.proc_pet == 1) ? kDeg2Rad * __ldg(a.latitude + k) : 0.0;
         r_sthresh = hm_recip_of(sthresh);
+        r_nd = hm_recip_of(a.nTstepDay);
         interc = S[(size_t)S_INTERC * N];
         snow = S[(size_t)S_SNOW * N] + 0.0; // a -0 ends with the first step's sum or zero
         seal = S[(size_t)S_SEAL * N];
@@ -211,13 +226,65 @@ template <bool LEAN> struct Surface {
         dd_thr_ok = !hm_isnan_i(dd_thr);  // prec <= NaN is false
     }
 
+    // pet, temp and prec of the step (mo_meteo_handler.f90:915-1285)
+    __device__ __forceinline__ void meteo(const CellArgs &a, const StepInfo si, const size_t f, const int k)
+    {
+        const int64_t N = a.n_cells;
+        const int month = si.month;
+        double pv = 0.0;
+        if (a.proc_pet == 0) {
+            pv = fasp * __ldg(a.pet + f);
+        } else if (a.proc_pet == -1) {
+            pv = petlai * __ldg(a.pet + f);
+        } else if constexpr (LEAN) {
+        } else if (a.proc_pet == 2) { // Rn = max(L1_netrad, 0), src/meteo/mo_meteo_handler.f90:1080-1085
+            const double rn = __ldg(a.netrad + f);
+            pv = pet_priestly(petlai, rn > 0.0 ? rn : 0.0, __ldg(a.temp + f));
+        } else if (a.proc_pet == 3) { // aeroResist / wind speed, eabs in kPa, :1087-1095
+            const double rn = __ldg(a.netrad + f);
+            pv = pet_penman(rn > 0.0 ? rn : 0.0, __ldg(a.temp + f), __ldg(a.eabs + f) / 1000.0,
+                            petlai / __ldg(a.wind + f), petsurf);
+        } else {
+            if (si.doy != cur_doy) {
+                cur_doy = si.doy;
+                rad = extraterr_rad_approx(cur_doy, lat_rad);
+            }
+            pv = fasp * pet_hargreaves(harsam, __ldg(a.temp + f), __ldg(a.tmax + f), __ldg(a.tmin + f), rad);
+        }
+        if (a.is_hourly) {
+            pet = pv;
+            temp = __ldg(a.temp + f);
+            prec = __ldg(a.pre + f);
+        } else if (a.w_pet) {
+            // temporal_disagg_meteo_weights (mo_meteo_temporal_tools.f90:32-50) with
+            // L1_*_weights(k, month, hour + 1), mo_meteo_handler.f90:1102-1107, 1183-1189,
+            // 1265-1270; temperature corrected by T0 = 273.15 K
+            const size_t wi = ((size_t)si.hour * 12 + (size_t)(month - 1)) * N + k;
+            pet = (pv + 0.0) * __ldg(a.w_pet + wi) - 0.0;
+            temp = (__ldg(a.temp + f) + kT0) * __ldg(a.w_temp + wi) - kT0;
+            prec = (__ldg(a.pre + f) + 0.0) * __ldg(a.w_pre + wi) - 0.0;
+        } else { // temporal_disagg_*_daynight, mo_meteo_temporal_tools.f90:66-161
+            const int mi = month - 1;
+            const double nd = a.nTstepDay;
+            if (nd > 1.0) {
+                const bool isday = (si.dflags & SF_ISDAY) != 0;
+                pet = hm_div_r(2.0 * pv * (isday ? a.tab.fday_pet[mi] : a.tab.fnight_pet[mi]), nd, r_nd);
+                temp = __ldg(a.temp + f) + (isday ? a.tab.fday_temp[mi] : a.tab.fnight_temp[mi]);
+                prec = hm_div_r(2.0 * __ldg(a.pre + f) * (isday ? a.tab.fday_prec[mi] : a.tab.fnight_prec[mi]), nd, r_nd);
+            } else {
+                pet = pv;
+                temp = __ldg(a.temp + f);
+                prec = __ldg(a.pre + f);
+            }
+        }
+    }
+
     // the step `si` of cell k of member m, forcing row `f` (an index); false:
     // the step's LAI entry is out of range (bounds-checked build)
     __device__ __forceinline__ bool step(const CellArgs &a, const double *P, const StepInfo si, const size_t f,
                                          const int m, const int k)
     {
         const int64_t N = a.n_cells;
-        const int month = si.month;
         bool ok = true;
         // the month (evap_coeff) and the LAI entry (iLAI: the month, or the
         // step's entry of a gridded LAI series) as one key: their parameters
@@ -245,55 +312,14 @@ template <bool LEAN> struct Surface {
             }
             r_imax = hm_recip_of(imax);
         }
-        // ---- meteo for the step (mo_meteo_handler.f90:915-1285) ----
-        double pv = 0.0;
-        if (a.proc_pet == 0) {
-            pv = fasp * __ldg(a.pet + f);
-        } else if (a.proc_pet == -1) {
-            pv = petlai * __ldg(a.pet + f);
-        } else if constexpr (LEAN) {
-        } else if (a.proc_pet == 2) { // Rn = max(L1_netrad, 0), src/meteo/mo_meteo_handler.f90:1080-1085
-            const double rn = __ldg(a.netrad + f);
-            pv = pet_priestly(petlai, rn > 0.0 ? rn : 0.0, __ldg(a.temp + f));
-        } else if (a.proc_pet == 3) { // aeroResist / wind speed, eabs in kPa, :1087-1095
-            const double rn = __ldg(a.netrad + f);
-            pv = pet_penman(rn > 0.0 ? rn : 0.0, __ldg(a.temp + f), __ldg(a.eabs + f) / 1000.0,
-                            petlai / __ldg(a.wind + f), petsurf);
-        } else {
-            if (si.doy != cur_doy) {
-                cur_doy = si.doy;
-                rad = extraterr_rad_approx(cur_doy, lat_rad);
-            }
-            pv = fasp * pet_hargreaves(harsam, __ldg(a.temp + f), __ldg(a.tmax + f), __ldg(a.tmin + f), rad);
+        bool fresh = true;
+        if constexpr (KEEP) {
+            const int day = key << 1 | (si.dflags & SF_ISDAY);
+            fresh = a.is_hourly || a.w_pet || f != cur_f || day != cur_day;
+            cur_f = f;
+            cur_day = day;
         }
-        double temp, prec;
-        if (a.is_hourly) {
-            pet = pv;
-            temp = __ldg(a.temp + f);
-            prec = __ldg(a.pre + f);
-        } else if (a.w_pet) {
-            // temporal_disagg_meteo_weights (mo_meteo_temporal_tools.f90:32-50) with
-            // L1_*_weights(k, month, hour + 1), mo_meteo_handler.f90:1102-1107, 1183-1189,
-            // 1265-1270; temperature corrected by T0 = 273.15 K
-            const size_t wi = ((size_t)si.hour * 12 + (size_t)(month - 1)) * N + k;
-            pet = (pv + 0.0) * __ldg(a.w_pet + wi) - 0.0;
-            temp = (__ldg(a.temp + f) + kT0) * __ldg(a.w_temp + wi) - kT0;
-            prec = (__ldg(a.pre + f) + 0.0) * __ldg(a.w_pre + wi) - 0.0;
-        } else { // temporal_disagg_*_daynight, mo_meteo_temporal_tools.f90:66-161
-            const int mi = month - 1;
-            const double nd = a.nTstepDay;
-            if (nd > 1.0) {
-                const bool isday = (si.dflags & SF_ISDAY) != 0;
-                pet = 2.0 * pv * (isday ? a.tab.fday_pet[mi] : a.tab.fnight_pet[mi]) / nd;
-                temp = __ldg(a.temp + f) + (isday ? a.tab.fday_temp[mi] : a.tab.fnight_temp[mi]);
-                prec = 2.0 * __ldg(a.pre + f) * (isday ? a.tab.fday_prec[mi] : a.tab.fnight_prec[mi]) / nd;
-            } else {
-                pet = pv;
-                temp = __ldg(a.temp + f);
-                prec = __ldg(a.pre + f);
-            }
-        }
-
+        if (fresh) meteo(a, si, f, k);
         // ---- canopy_interc, mo_canopy_interc.f90:75-133 ----
         // Branches that only pick between values are written as hm_sel (an
         // integer select of the bits): a double select or a merge of doubles
@@ -432,6 +458,11 @@ struct Ground {
         return q;
     }
 };
+
+__host__ inline bool cell_chain_lean(const CellArgs &a)
+{
+    return (a.proc_pet == 0 || a.proc_pet == -1) && (a.proc_sm == 1 || a.proc_sm == 4);
+}
 
 // LEAN: compiled for PET input (cases -1, 0) and the Feddes stress (soil-moisture
 // cases 1, 4) only -- the configurations of the throughput workloads -- so that
@@ -897,8 +928,7 @@ template <int MINB, bool FLUX = false>
 cudaError_t launch_cell_chain_variant(const CellArgs &a, int H, cudaStream_t s)
 {
     if constexpr (!FLUX) {
-        const bool lean = (a.proc_pet == 0 || a.proc_pet == -1) && (a.proc_sm == 1 || a.proc_sm == 4);
-        if (lean) return launch_cell_chain_h<MINB, false, true>(a, H, s);
+        if (cell_chain_lean(a)) return launch_cell_chain_h<MINB, false, true>(a, H, s);
     }
     return launch_cell_chain_h<MINB, FLUX, false>(a, H, s);
 }

@@ -46,6 +46,7 @@ cudaError_t launch_bc_selftest(cudaStream_t s);
 cudaError_t bc_take_cell_chain(unsigned long long *out);
 cudaError_t bc_take_cell_chain_o6(unsigned long long *out);
 cudaError_t bc_take_cell_chain_o8(unsigned long long *out);
+cudaError_t bc_take_cell_chain_small(unsigned long long *out);
 cudaError_t bc_take_routing(unsigned long long *out);
 cudaError_t bc_take_mpr(unsigned long long *out);
 } // namespace mhm
@@ -193,6 +194,7 @@ struct mhm_ctx {
     int32_t lai_mode = 0, n_lai = 0;
     DevBuf<double> lai_series;
     int32_t cell_occ = 4;  // cell-chain register variant: resident blocks per SM (4, 6, 8)
+    int32_t cell_small = 1; // launches of few cells take the kernel of cell_chain_small.cu
     int32_t chunk_cap = 0; // most time steps per chunk (0: the device-memory budget decides)
     // routing case 2: per-member routing time step [s] and the link lengths
     std::vector<double> ts_rout, length_h;
@@ -742,6 +744,7 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
         int v = std::atoi(s);
         if (v == 4 || v == 6 || v == 8) ctx->cell_occ = v;
     }
+    if (const char *s = std::getenv("MHM_CELL_SMALL")) ctx->cell_small = std::atoi(s) != 0;
     if (const char *s = std::getenv("MHM_ROUTE_POLLS")) ctx->route_polls = std::max(0, std::atoi(s));
     if (const char *s = std::getenv("MHM_ROUTE_CLUSTER")) {
         int v = std::atoi(s);
@@ -1460,6 +1463,7 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         a.tab = ctx->tab;
         a.nonfinite = ctx->nonfinite.p;
         a.n_horizons = H;
+        a.small_ok = ctx->cell_small;
         if (ctx->lai_mode < 0) {
             a.lai_series = ctx->lai_series.p;
             a.n_lai = ctx->n_lai;
@@ -1755,7 +1759,7 @@ static int take_bounds_status(mhm_ctx *ctx, int32_t *site, int64_t *index)
     if (index) *index = 0;
     if (!kBoundsChecked) return MHM_OK;
     cudaError_t (*const readers[])(unsigned long long *) = {bc_take_cell_chain, bc_take_cell_chain_o6,
-                                                            bc_take_cell_chain_o8, bc_take_routing, bc_take_mpr};
+                                                            bc_take_cell_chain_o8, bc_take_cell_chain_small, bc_take_routing, bc_take_mpr};
     unsigned long long first = 0;
     for (auto rd : readers) {
         unsigned long long v = 0;

@@ -133,7 +133,8 @@ struct CellArgs {
     // per-member failure flag: bit 0 set when the member's total runoff of a
     // step or a state at the chunk's end is not finite (nullptr = not checked)
     int32_t *nonfinite;
-    int32_t n_horizons; // the context's horizon count (read by the fused multi-context launch)
+    int32_t n_horizons; // the context's horizon count (read by the fused and the small launch)
+    int32_t small_ok;   // a launch of few cells may take the small launch's kernel
     // extents the bounds-checked build tests its data-derived indexes against:
     // forcing rows from row_base (or window rows in member mode) and, in member
     // mode, the rows of the member step table
