@@ -33,9 +33,9 @@ cudaError_t launch_route_flow(const RouteArgs &a, int round, cudaStream_t s);
 cudaError_t launch_qmod_step(const QmodStepArgs &a, cudaStream_t s);
 cudaError_t launch_gauge_gather(const GaugeArgs &a, cudaStream_t s);
 cudaError_t launch_qrouted(const QroutArgs &a, cudaStream_t s);
-cudaError_t launch_reg_rout(int n_links, const double *p5, double ss_max, double TS, const double *length,
-                            const double *slope, const double *ffp, const int32_t *link_pos, double *C1,
-                            double *C2, cudaStream_t s);
+cudaError_t launch_reg_rout(int n_members, int n_links, int n_nodes, const double *p5, int p5_stride, double ss_max,
+                            double TS, const double *length, const double *slope, const double *ffp,
+                            const int32_t *link_pos, double *C1, double *C2, cudaStream_t s);
 cudaError_t launch_hmath_eval(int op, int64_t n, const double *x, const double *y, double *out, cudaStream_t s);
 cudaError_t launch_fp64_probe(int64_t iters, int blocks, int threads, double *sink, cudaStream_t s);
 cudaError_t launch_mpr(const MprArgs &a, cudaStream_t s);
@@ -1071,7 +1071,7 @@ int mhm_set_routing_params(mhm_ctx *ctx, int32_t m, const double *p5)
     const size_t L = ctx->L;
     CK(cudaMemcpyAsync(ctx->rout_p5.p + 5 * m, p5, 5 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream), "p5");
     Bracket br(ctx, 2, ctx->stream);
-    CK(launch_reg_rout(ctx->n_links, ctx->rout_p5.p + 5 * m, ctx->ss_max, (double)ctx->timestep, ctx->length.p,
+    CK(launch_reg_rout(1, ctx->n_links, ctx->L, ctx->rout_p5.p + 5 * m, 5, ctx->ss_max, (double)ctx->timestep, ctx->length.p,
                        ctx->slope.p, ctx->ffp.p, ctx->link_pos.p, ctx->C1.p + m * L, ctx->C2.p + m * L,
                        ctx->stream),
        "reg_rout");
@@ -2660,16 +2660,11 @@ int mhm_mpr(mhm_ctx *ctx, int32_t member0, int32_t n, const double *gammas, int3
     g_launches += 2;
     if (ctx->proc_rout == 1 && ctx->n_links > 0) {
         const size_t L = ctx->L;
-        for (int32_t i = 0; i < n; ++i) {
-            const int32_t mm = member0 + i;
-            const double *p5 = ctx->mpr_gamma.p + (size_t)i * n_gamma + off.routing;
-            CK(cudaMemcpyAsync(ctx->rout_p5.p + 5 * mm, p5, 5 * sizeof(double), cudaMemcpyDeviceToDevice, s), "p5");
-            CK(launch_reg_rout(ctx->n_links, ctx->rout_p5.p + 5 * mm, ctx->ss_max, (double)ctx->timestep,
-                               ctx->length.p, ctx->slope.p, ctx->ffp.p, ctx->link_pos.p, ctx->C1.p + mm * L,
-                               ctx->C2.p + mm * L, s),
-               "reg_rout");
-            g_launches++;
-        }
+        CK(launch_reg_rout(n, ctx->n_links, ctx->L, ctx->mpr_gamma.p + off.routing, n_gamma, ctx->ss_max,
+                           (double)ctx->timestep, ctx->length.p, ctx->slope.p, ctx->ffp.p, ctx->link_pos.p,
+                           ctx->C1.p + member0 * L, ctx->C2.p + member0 * L, s),
+           "reg_rout");
+        g_launches++;
     }
     if (ctx->proc_rout == 2)
         for (int32_t i = 0; i < n; ++i)
@@ -2785,12 +2780,9 @@ int mhm_mpr_noalloc(mhm_ctx *ctx, int32_t member, const double *gamma, int32_t n
     g_launches += 2;
     if (ctx->proc_rout == 1 && ctx->n_links > 0) {
         const size_t L = ctx->L;
-        CK(cudaMemcpyAsync(ctx->rout_p5.p + 5 * member, d_gamma + off.routing, 5 * sizeof(double),
-                           cudaMemcpyDeviceToDevice, s),
-           "p5");
-        CK(launch_reg_rout(ctx->n_links, ctx->rout_p5.p + 5 * member, ctx->ss_max, (double)ctx->timestep,
-                           ctx->length.p, ctx->slope.p, ctx->ffp.p, ctx->link_pos.p, ctx->C1.p + member * L,
-                           ctx->C2.p + member * L, s),
+        CK(launch_reg_rout(1, ctx->n_links, ctx->L, d_gamma + off.routing, n_gamma, ctx->ss_max,
+                           (double)ctx->timestep, ctx->length.p, ctx->slope.p, ctx->ffp.p, ctx->link_pos.p,
+                           ctx->C1.p + member * L, ctx->C2.p + member * L, s),
            "reg_rout");
         g_launches++;
     }

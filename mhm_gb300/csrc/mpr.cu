@@ -18,6 +18,7 @@
 
 #include "hmath.h"
 #include "bounds.cuh"
+#include "fp64i.h"
 #include "mhm_kernels.cuh"
 #include "mpr_host.h"
 
@@ -82,233 +83,218 @@ __device__ double pwp(double n, double alpha, double ths)
 // the pair's L0 quantities, then mpr_SMhorizons (src/MPR/mo_mpr_smhorizons.f90:
 // 340-582) for each model horizon; harmonic-mean operands are stored as the
 // reciprocals the upscaling sums.
-__device__ void soil_row(const MprArgs &a, const double *g, int s, int l, double *row)
+//
+// What bounds it: one lane's chain of eleven elementary functions, then two
+// powers and five divisions (9,000-12,000 cycles).  So a row has 16 lanes: a
+// lane per soil horizon, then a lane per model horizon and one for the
+// column's quantities.  30 rows, cold: 89 us with one thread a row, 41 us here (one
+// copy of each function instead of the inlined ones changed nothing).
+constexpr int kRowLanes = kMprMaxSoilHor, kTableRows = 4;
+static_assert(kRowLanes == 16 && kMaxHorizons < kRowLanes, "a row's lanes are half a warp, the last for the column");
+struct SoilRow {
+    double ths[kMprMaxSoilHor], thfc[kMprMaxSoilHor], thpw[kMprMaxSoilHor], ks[kMprMaxSoilHor], db[kMprMaxSoilHor];
+};
+
+__device__ void soil_row(const MprArgs &a, const double *g, int s, int l, int lane, SoilRow &w, double *row)
 {
     const int H = a.H, mh = a.max_hor, nh = a.n_hor[s], nt = a.n_till[s];
     const double *ps = g + a.off.soil;
-    const double om_forest = (a.proc_sm <= 2) ? ps[2] + ps[0] : ps[0];
-    const double pom = (l == 0) ? om_forest : (l == 1) ? ps[1] : ps[2];
-    double ths[kMprMaxSoilHor], thfc[kMprMaxSoilHor], thpw[kMprMaxSoilHor], ks[kMprMaxSoilHor],
-        db[kMprMaxSoilHor];
-    for (int j = 0; j < nh; ++j) {
+    if (lane < nh) {
+        const int j = lane;
+        const double om_forest = (a.proc_sm <= 2) ? ps[2] + ps[0] : ps[0];
+        const double pom = (l == 0) ? om_forest : (l == 1) ? ps[1] : ps[2];
         const double sand = a.sand[s * mh + j], clay = a.clay[s * mh + j], dbm = a.dbm[s * mh + j];
-        double k = hydro_cond(ps + 9, sand, clay), n, alpha;
+        double k = hydro_cond(ps + 9, sand, clay), n, alpha, db = dbm, ths;
         if (j < nt) {
             const double pm = 100.0 - pom;
-            db[j] = 100.0 / ((pom / kBulkDensOrgMatter) + (pm / dbm));
-            k = k * (dbm / db[j]);
-            genuchten(ps + 3, sand, clay, db[j], ths[j], n, alpha);
-        } else {
-            db[j] = dbm;
-            genuchten(ps + 3, sand, clay, dbm, ths[j], n, alpha);
+            db = hm_div(100.0, hm_div(pom, kBulkDensOrgMatter) + hm_div(pm, dbm));
+            k = k * hm_div(dbm, db);
         }
-        ks[j] = k;
-        thfc[j] = field_cap(k, ths[j], n);
-        thpw[j] = pwp(n, alpha, ths[j]);
+        genuchten(ps + 3, sand, clay, db, ths, n, alpha);
+        w.db[j] = db;
+        w.ks[j] = k;
+        w.ths[j] = ths;
+        w.thfc[j] = field_cap(k, ths, n);
+        w.thpw[j] = pwp(n, alpha, ths);
     }
-    // Ks variabilities over the column (:330-352)
-    double kh = 0.0, kv = 0.0, fc = 0.0, tot = 0.0;
-    for (int j = 0; j < nh; ++j) {
-        kh = kh + ths[j] * ks[j];
-        kv = kv + ths[j] / ks[j];
-        fc = fc + thfc[j];
-        tot = tot + ths[j];
+    __syncwarp();
+    if (lane == kRowLanes - 1) {
+        // Ks variabilities over the column (:330-352)
+        double kh = 0.0, kv = 0.0, fc = 0.0, tot = 0.0;
+        for (int j = 0; j < nh; ++j) {
+            kh = kh + w.ths[j] * w.ks[j];
+            kv = kv + hm_div(w.ths[j], w.ks[j]);
+            fc = fc + w.thfc[j];
+            tot = tot + w.ths[j];
+        }
+        const double sms_fc = hm_div(tot - fc, tot);
+        const double ksvar_h = hm_div(hm_div(kh, tot), ps[12]);
+        const double ksvar_v = hm_div(hm_div(tot, kv), ps[12]);
+        const double *pi = g + a.off.interflow, *pp = g + a.off.perc;
+        row[5 * H + 0] = pi[0] * sms_fc;                                                   // mpr_runoff HL1 operand
+        row[5 * H + 1] = pi[3] * (1.0 + ksvar_h);                                          // K1 soil term
+        row[5 * H + 2] = pi[4] * hm_div(1.0, ksvar_h) * hm_div(1.0, 1.0 + sms_fc);         // alpha operand
+        row[5 * H + 3] = hm_div(pp[0] * (1.0 + sms_fc), 1.0 + ksvar_v);                    // karstic_layer Kp operand
     }
-    const double sms_fc = (tot - fc) / tot;
-    const double ksvar_h = kh / tot / ps[12];
-    const double ksvar_v = tot / kv / ps[12];
+    if (lane >= H) return;
 
     // horizons (mpr_SMhorizons); its 4 or 8 parameters follow the first 13
+    const int h = lane;
     const double *p2 = ps + 13;
-    const double rc_forest = p2[0], rc_imp = p2[1];
-    double rc_perv = 0.0, rc_sand = 0.0, rc_clay = 0.0, fcmin = 0.0, fcmax = 0.0;
-    if (a.proc_sm <= 2) {
-        rc_perv = p2[0] - p2[2];
-    } else {
-        rc_perv = p2[2];
-        rc_sand = p2[5] - p2[4];
-        rc_clay = p2[5];
-        fcmin = p2[6];
-        fcmax = p2[6] + p2[7];
-    }
-    for (int h = 0; h < H; ++h) {
-        const double *wd = a.Wd + ((size_t)s * H + h) * mh;
-        double a1 = 0.0, b1 = 0.0;
+    const double *wd = a.Wd + ((size_t)s * H + h) * mh;
+    double a1 = 0.0, b1 = 0.0;
+    for (int j = 0; j < nt; ++j)
+        if (wd[j] > 0.0) a1 = a1 + w.db[j] * wd[j];
+    for (int j = nt; j < nh; ++j)
+        if (wd[j] >= 0.0) b1 = b1 + w.db[j] * wd[j];
+    const double bd = a1 + b1;
+    double sums[3];
+    const double *th[3] = {w.ths, w.thfc, w.thpw};
+    for (int q = 0; q < 3; ++q) {
+        double x = 0.0, y = 0.0;
         for (int j = 0; j < nt; ++j)
-            if (wd[j] > 0.0) a1 = a1 + db[j] * wd[j];
+            if (wd[j] > 0.0) x = x + th[q][j] * wd[j];
         for (int j = nt; j < nh; ++j)
-            if (wd[j] >= 0.0) b1 = b1 + db[j] * wd[j];
-        const double bd = a1 + b1;
-        double sums[3];
-        const double *th[3] = {ths, thfc, thpw};
-        for (int q = 0; q < 3; ++q) {
-            double x = 0.0, y = 0.0;
-            for (int j = 0; j < nt; ++j)
-                if (wd[j] > 0.0) x = x + th[q][j] * wd[j];
-            for (int j = nt; j < nh; ++j)
-                if (wd[j] > 0.0) y = y + th[q][j] * wd[j];
-            sums[q] = x + y;
-        }
-        double dpth_f = 0.0, dpth_t = a.hd[h];
-        if (h > 0 && h < H - 1) dpth_f = a.hd[h - 1];
-        double dpth_t_roots = dpth_t;
-        if (h == H - 1) {
-            dpth_f = a.hd[H - 2];
-            dpth_t = a.rz[s];               // this cell's own soil
-            dpth_t_roots = a.dpth_t_last;   // what the root loop sees afterwards
-        }
-        const double sms = sums[0] * (dpth_t - dpth_f);
-        const double fcv = sums[1] * (dpth_t - dpth_f);
-        const double pwv = sums[2] * (dpth_t - dpth_f);
-        double c;
-        if (l == 0) {
-            c = rc_forest;
-        } else if (l == 1) {
-            c = rc_imp;
-        } else if (a.proc_sm <= 2) {
-            c = rc_perv;
-        } else {
-            double fcn = (((fcv / (dpth_t_roots - dpth_f)) - fcmin) / (fcmax - fcmin));
-            if (fcn < 0.0)
-                fcn = 0.0;
-            else if (fcn > 1.0)
-                fcn = 1.0;
-            c = (fcn * rc_clay) + ((1.0 - fcn) * rc_sand);
-        }
-        const double fr = (1.0 - hm_pow(c, dpth_t_roots * 0.1)) - (1.0 - hm_pow(c, dpth_f * 0.1));
-        row[MT_INV_SMS * H + h] = 1.0 / sms;
-        row[MT_INV_BETA * H + h] = 1.0 / (bd * p2[3]);
-        row[MT_INV_PW * H + h] = 1.0 / pwv;
-        row[MT_INV_FC * H + h] = 1.0 / fcv;
-        row[MT_INV_FROOTS * H + h] = 1.0 / fr;
+            if (wd[j] > 0.0) y = y + th[q][j] * wd[j];
+        sums[q] = x + y;
     }
-    const double *pi = g + a.off.interflow, *pp = g + a.off.perc;
-    row[5 * H + 0] = pi[0] * sms_fc;                                      // mpr_runoff HL1 operand
-    row[5 * H + 1] = pi[3] * (1.0 + ksvar_h);                             // K1 soil term
-    row[5 * H + 2] = pi[4] * (1.0 / ksvar_h) * (1.0 / (1.0 + sms_fc));    // alpha operand
-    row[5 * H + 3] = pp[0] * (1.0 + sms_fc) / (1.0 + ksvar_v);            // karstic_layer Kp operand
+    double dpth_f = 0.0, dpth_t = a.hd[h];
+    if (h > 0 && h < H - 1) dpth_f = a.hd[h - 1];
+    double dpth_t_roots = dpth_t;
+    if (h == H - 1) {
+        dpth_f = a.hd[H - 2];
+        dpth_t = a.rz[s];               // this cell's own soil
+        dpth_t_roots = a.dpth_t_last;   // what the root loop sees afterwards
+    }
+    const double sms = sums[0] * (dpth_t - dpth_f);
+    const double fcv = sums[1] * (dpth_t - dpth_f);
+    const double pwv = sums[2] * (dpth_t - dpth_f);
+    double c;
+    if (l == 0) {
+        c = p2[0];
+    } else if (l == 1) {
+        c = p2[1];
+    } else if (a.proc_sm <= 2) {
+        c = p2[0] - p2[2];
+    } else {
+        const double rc_sand = p2[5] - p2[4], rc_clay = p2[5], fcmin = p2[6], fcmax = p2[6] + p2[7];
+        double fcn = hm_div(hm_div(fcv, dpth_t_roots - dpth_f) - fcmin, fcmax - fcmin);
+        if (fcn < 0.0)
+            fcn = 0.0;
+        else if (fcn > 1.0)
+            fcn = 1.0;
+        c = (fcn * rc_clay) + ((1.0 - fcn) * rc_sand);
+    }
+    const double fr = (1.0 - hm_pow(c, dpth_t_roots * 0.1)) - (1.0 - hm_pow(c, dpth_f * 0.1));
+    row[MT_INV_SMS * H + h] = hm_div(1.0, sms);
+    row[MT_INV_BETA * H + h] = hm_div(1.0, bd * p2[3]);
+    row[MT_INV_PW * H + h] = hm_div(1.0, pwv);
+    row[MT_INV_FC * H + h] = hm_div(1.0, fcv);
+    row[MT_INV_FROOTS * H + h] = hm_div(1.0, fr);
 }
 
-// grid (ceil(rows / 64), members): soil rows, then (proc_pet = -1 with class
-// LAI) the reciprocal LAI correction factors of pet_correctbyLAI
-// (src/MPR/mo_mpr_pet.f90:60-140) per (land cover, LAI class, month)
-__global__ void __launch_bounds__(64) mpr_table_kernel(MprArgs a)
+// grid (ceil(n_keys / 4) + ceil(LAI entries / 64), members): soil rows, then
+// (proc_pet = -1 with class LAI) the reciprocal LAI correction factors of
+// pet_correctbyLAI (src/MPR/mo_mpr_pet.f90:60-140) per (land cover, LAI class,
+// month)
+__global__ void __launch_bounds__(kTableRows * kRowLanes) mpr_table_kernel(MprArgs a)
 {
-    const int m = blockIdx.y;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ SoilRow rows[kTableRows];
+    const int m = blockIdx.y, r = threadIdx.x / kRowLanes;
+    const int row_blocks = (a.n_keys + kTableRows - 1) / kTableRows;
     const double *g = a.gamma + (size_t)m * a.n_gamma;
     const int ts = mpr_table_stride(a.H);
-    if (t < a.n_keys) {
-        soil_row(a, g, t / 3, t % 3, a.table + ((size_t)m * a.n_keys + t) * ts);
+    if ((int)blockIdx.x < row_blocks) {
+        const int t = (int)blockIdx.x * kTableRows + r;
+        if (t >= a.n_keys) return;
+        soil_row(a, g, t / 3, t % 3, threadIdx.x % kRowLanes, rows[r], a.table + ((size_t)m * a.n_keys + t) * ts);
         return;
     }
-    const int u = t - a.n_keys;
-    if (a.proc_pet != -1 || a.n_lai_classes == 0 || u >= 3 * a.n_lai_classes * 12) return;
+    const int u = ((int)blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
+    if (a.proc_pet != -1 || u >= 3 * a.n_lai_classes * 12) return;
     const int l = u / (a.n_lai_classes * 12), c = (u / 12) % a.n_lai_classes, mo = u % 12;
     const double *p = g + a.off.pet;
     const double base = (l == 0) ? p[0] : (l == 1) ? p[1] : p[2];
     const double f = base + (p[3] * (1.0 - hm_exp(p[4] * a.lai_lut[c * 12 + mo])));
-    a.petlai[(size_t)m * 3 * a.n_lai_classes * 12 + u] = 1.0 / f;
+    a.petlai[(size_t)m * 3 * a.n_lai_classes * 12 + u] = hm_div(1.0, f);
 }
 
-// grid (ceil(n1 / 128), members): one thread per L1 cell
-__global__ void __launch_bounds__(128) mpr_upscale_kernel(MprArgs a)
+// The arithmetic mean's division by the number of sub-cells, the same for all
+// of a cell's means
+struct Mean {
+    double dn;
+    uint64_t inv;
+    __device__ explicit Mean(double n) : dn(n), inv(hm_recip_of(n)) {}
+    __device__ double operator()(double sum) const { return hm_div_r(sum, dn, inv); }
+};
+
+// One soil horizon of a cell: harmonic means (upscale_harmonic_mean,
+// src/MPR/mo_upscaling_operators.f90:369-432), then the limits of
+// mpr_SMhorizons (src/MPR/mo_mpr_smhorizons.f90:712-737).  Returns the root
+// fraction before its normalisation.
+__device__ double upscale_horizon(const MprArgs &a, int h, int k, int ns, const double *tab, double *out)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n1) return;
-    const int m = blockIdx.y, H = a.H, ts = mpr_table_stride(H);
+    const int H = a.H, ts = mpr_table_stride(H);
     const size_t N = a.n1;
-    const double *g = a.gamma + (size_t)m * a.n_gamma;
-    const double *tab = a.table + (size_t)m * a.n_keys * ts;
-    double *out = a.params + (size_t)m * a.member_stride;
-    const int ns = a.nsub[k];
-    const double dn = (double)ns;
     const uint32_t *code = a.code + k;
-    const double *se = a.se + k, *asp = a.asp + k;
-
-    // soil horizons: harmonic means (upscale_harmonic_mean,
-    // src/MPR/mo_upscaling_operators.f90:369-432), then the limits and the
-    // root normalisation of mpr_SMhorizons (src/MPR/mo_mpr_smhorizons.f90:712-737)
-    double froots[kMaxHorizons];
-    for (int h = 0; h < H; ++h) {
-        double s_sms = 0.0, s_beta = 0.0, s_pw = 0.0, s_fc = 0.0, s_fr = 0.0;
-        for (int j = 0; j < ns; ++j) {
-            const uint32_t key = __ldg(code + (size_t)j * N) & kMprKeyMask;
-            if (!bc_ok(BC_MPR_KEY, key, a.n_keys)) continue;
-            const double *row = tab + (size_t)key * ts;
-            s_sms = s_sms + __ldg(row + MT_INV_SMS * H + h);
-            s_beta = s_beta + __ldg(row + MT_INV_BETA * H + h);
-            s_pw = s_pw + __ldg(row + MT_INV_PW * H + h);
-            s_fc = s_fc + __ldg(row + MT_INV_FC * H + h);
-            s_fr = s_fr + __ldg(row + MT_INV_FROOTS * H + h);
-        }
-        double sms = dn / s_sms, fc = dn / s_fc, pw = dn / s_pw;
-        froots[h] = dn / s_fr;
-        if (fc > sms) fc = sms - 0.01 * sms;
-        if (pw > fc) pw = fc - 0.01 * fc;
-        if (sms < 0.0) sms = 0.0001;
-        if (fc < 0.0) fc = 0.0001;
-        if (pw < 0.0) pw = 0.0001;
-        out[(size_t)(P_HORIZON + 1 * H + h) * N + k] = sms;
-        out[(size_t)(P_HORIZON + 2 * H + h) * N + k] = fc;
-        out[(size_t)(P_HORIZON + 3 * H + h) * N + k] = pw;
-        out[(size_t)(P_HORIZON + 4 * H + h) * N + k] = dn / s_beta;
-    }
-    double ftot = 0.0;
-    for (int h = 0; h < H; ++h)
-        if (froots[h] > 0.0) ftot = ftot + froots[h];
-    for (int h = 0; h < H; ++h)
-        out[(size_t)(P_HORIZON + h) * N + k] = (ftot > 0.0) ? froots[h] / ftot : 0.0;
-
-    // arithmetic means (upscale_arithmetic_mean, :266-329) of mpr_runoff
-    // (src/MPR/mo_mpr_runoff.f90:141-191), karstic_layer (Kp), baseflow_param
-    // and pet_correctbyASP (src/MPR/mo_mpr_pet.f90:236-272)
-    const double *pi = g + a.off.interflow, *pp = g + a.off.pet, *geo = g + a.off.geo;
-    const bool asp_on = (a.proc_pet == 0 || a.proc_pet == 1);
-    const double tmax = pp[0] + pp[1];
-    const double slope_lo = asp_on ? (tmax - pp[0]) / pp[2] : 0.0;
-    const double slope_hi = asp_on ? (tmax - pp[0]) / (360.0 - pp[2]) : 0.0;
-    double s_hl1 = 0.0, s_k0 = 0.0, s_k1 = 0.0, s_alpha = 0.0, s_kp = 0.0, s_k2 = 0.0, s_asp = 0.0;
+    const double dn = (double)ns;
+    double s_sms = 0.0, s_beta = 0.0, s_pw = 0.0, s_fc = 0.0, s_fr = 0.0;
     for (int j = 0; j < ns; ++j) {
-        const uint32_t c = __ldg(code + (size_t)j * N);
+        const uint32_t key = __ldg(code + (size_t)j * N) & kMprKeyMask;
+        if (!bc_ok(BC_MPR_KEY, key, a.n_keys)) continue;
+        const double *row = tab + (size_t)key * ts;
+        s_sms = s_sms + __ldg(row + MT_INV_SMS * H + h);
+        s_beta = s_beta + __ldg(row + MT_INV_BETA * H + h);
+        s_pw = s_pw + __ldg(row + MT_INV_PW * H + h);
+        s_fc = s_fc + __ldg(row + MT_INV_FC * H + h);
+        s_fr = s_fr + __ldg(row + MT_INV_FROOTS * H + h);
+    }
+    double sms = hm_div(dn, s_sms), fc = hm_div(dn, s_fc), pw = hm_div(dn, s_pw);
+    if (fc > sms) fc = sms - 0.01 * sms;
+    if (pw > fc) pw = fc - 0.01 * fc;
+    if (sms < 0.0) sms = 0.0001;
+    if (fc < 0.0) fc = 0.0001;
+    if (pw < 0.0) pw = 0.0001;
+    out[(size_t)(P_HORIZON + 1 * H + h) * N + k] = sms;
+    out[(size_t)(P_HORIZON + 2 * H + h) * N + k] = fc;
+    out[(size_t)(P_HORIZON + 3 * H + h) * N + k] = pw;
+    out[(size_t)(P_HORIZON + 4 * H + h) * N + k] = hm_div(dn, s_beta);
+    return hm_div(dn, s_fr);
+}
+
+// Arithmetic means (upscale_arithmetic_mean, :266-329): the thresholds and
+// recession constants of mpr_runoff (src/MPR/mo_mpr_runoff.f90:141-191) and
+// baseflow_param; then the values that need no sub-cells: snow
+// (snow_acc_melt_param, src/MPR/mo_multi_param_reg.f90:800-852), sealed
+// threshold, karst loss (karstic_layer, :1032) and Jarvis threshold
+__device__ void upscale_recession(const MprArgs &a, const double *g, int k, int ns, const double *tab, double *out)
+{
+    const int H = a.H, ts = mpr_table_stride(H);
+    const size_t N = a.n1;
+    const double *pi = g + a.off.interflow, *geo = g + a.off.geo;
+    const double p1 = pi[1], p2 = pi[2];
+    double s_k0 = 0.0, s_k1 = 0.0, s_k2 = 0.0;
+    for (int j = 0; j < ns; ++j) {
+        const uint32_t c = __ldg(a.code + k + (size_t)j * N);
         if (!bc_ok(BC_MPR_KEY, c & kMprKeyMask, a.n_keys) ||
             !bc_ok(BC_MPR_GEO, (long long)(c >> 24), (long long)a.n_gamma - a.off.geo))
             continue;
-        const double *row = tab + (size_t)(c & kMprKeyMask) * ts;
-        const double sej = __ldg(se + (size_t)j * N);
-        s_hl1 = s_hl1 + __ldg(row + 5 * H + 0);
-        double t0 = pi[1] * (2.0 - sej);
-        if (c & kMprForest) t0 = t0 * pi[2];
+        const double t1 = p1 * (2.0 - __ldg(a.se + k + (size_t)j * N));
+        double t0 = t1;
+        if (c & kMprForest) t0 = t0 * p2;
         s_k0 = s_k0 + t0;
-        s_k1 = s_k1 + (pi[1] * (2.0 - sej) + __ldg(row + 5 * H + 1));
-        s_alpha = s_alpha + __ldg(row + 5 * H + 2);
-        s_kp = s_kp + __ldg(row + 5 * H + 3);
-        s_k2 = s_k2 + geo[c >> 24];
-        if (asp_on) {
-            const double x = __ldg(asp + (size_t)j * N);
-            // northern cells: the low branch below the threshold aspect;
-            // southern cells: the mirrored assignment
-            const bool low = ((c & kMprNorth) != 0) == (x < pp[2]);
-            s_asp = s_asp + (low ? pp[0] + slope_lo * x : pp[0] + slope_hi * (360.0 - x));
-        }
+        s_k1 = s_k1 + (t1 + __ldg(tab + (size_t)(c & kMprKeyMask) * ts + 5 * H + 1));
+        s_k2 = s_k2 + __ldg(geo + (c >> 24));
     }
-    double k0 = s_k0 / dn, k1 = s_k1 / dn, kp = s_kp / dn, k2 = s_k2 / dn;
+    const Mean mean((double)ns);
+    double k0 = mean(s_k0), k1 = mean(s_k1), k2 = mean(s_k2);
     if (k0 < 1.0) k0 = 1.0;
     if (k1 < 2.0) k1 = 2.0;
     if (k0 > k1) k0 = k1;
-    if (kp < 2.0) kp = 2.0;
     if (k2 < k1) k2 = k1; // src/MPR/mo_multi_param_reg.f90:618
-    out[(size_t)P_UTHRESH * N + k] = s_hl1 / dn;
     out[(size_t)P_K0 * N + k] = k0;
     out[(size_t)P_K1 * N + k] = k1;
-    out[(size_t)P_ALPHA * N + k] = s_alpha / dn;
-    out[(size_t)P_KP * N + k] = kp;
     out[(size_t)P_K2 * N + k] = k2;
-    out[(size_t)P_FASP * N + k] = asp_on ? s_asp / dn : 0.0;
-    out[(size_t)P_HARSAM * N + k] = (a.proc_pet == 1) ? pp[3] : 0.0;
-
-    // land-cover fractions, snow (snow_acc_melt_param, :800-852), sealed
-    // threshold, karst loss (karstic_layer, :1032) and Jarvis threshold
     const double *psn = g + a.off.snow;
     const double ff = a.f_forest[k], fs = a.f_sealed[k], fp = a.f_perm[k];
     const double ddf_f = psn[1], ddf_i = psn[1] + psn[3] + psn[2], ddf_p = psn[1] + psn[3];
@@ -322,33 +308,92 @@ __global__ void __launch_bounds__(128) mpr_upscale_kernel(MprArgs a)
     out[(size_t)P_KARST * N + k] = 1.0 - (a.f_kar[k] * g[a.off.perc + 1]);
     out[(size_t)P_JARVIS * N + k] =
         (a.proc_sm == 2 || a.proc_sm == 3) ? g[a.off.soil + a.off.n_soil_params - 1] : 0.0;
+}
 
-    // canopy_intercept_param (src/MPR/mo_multi_param_reg.f90:1132-1152) and
-    // pet_correctbyLAI, per LAI entry (12 monthly slots or a gridded series:
-    // the reference loops over size(LAI0, 2), :1142)
-    const double gi = g[a.off.interc];
-    const size_t slots = (size_t)a.max_sub * N;
+// ... interflow threshold and exponent, percolation (karstic_layer), and
+// pet_correctbyASP (src/MPR/mo_mpr_pet.f90:236-272)
+__device__ void upscale_aspect(const MprArgs &a, const double *g, int k, int ns, const double *tab, double *out)
+{
+    const int H = a.H, ts = mpr_table_stride(H);
+    const size_t N = a.n1;
+    const double *pp = g + a.off.pet;
+    const bool asp_on = (a.proc_pet == 0 || a.proc_pet == 1);
+    const double tmax = pp[0] + pp[1];
+    const double slope_lo = asp_on ? (tmax - pp[0]) / pp[2] : 0.0;
+    const double slope_hi = asp_on ? (tmax - pp[0]) / (360.0 - pp[2]) : 0.0;
+    double s_hl1 = 0.0, s_alpha = 0.0, s_kp = 0.0, s_asp = 0.0;
+    for (int j = 0; j < ns; ++j) {
+        const uint32_t c = __ldg(a.code + k + (size_t)j * N);
+        if (!bc_ok(BC_MPR_KEY, c & kMprKeyMask, a.n_keys) ||
+            !bc_ok(BC_MPR_GEO, (long long)(c >> 24), (long long)a.n_gamma - a.off.geo))
+            continue;
+        const double *row = tab + (size_t)(c & kMprKeyMask) * ts + 5 * H;
+        s_hl1 = s_hl1 + __ldg(row);
+        s_alpha = s_alpha + __ldg(row + 2);
+        s_kp = s_kp + __ldg(row + 3);
+        if (asp_on) {
+            const double x = __ldg(a.asp + k + (size_t)j * N);
+            // northern cells: the low branch below the threshold aspect;
+            // southern cells: the mirrored assignment
+            const bool low = ((c & kMprNorth) != 0) == (x < pp[2]);
+            s_asp = s_asp + (pp[0] + hm_sel(low, slope_lo, slope_hi) * hm_sel(low, x, 360.0 - x));
+        }
+    }
+    const Mean mean((double)ns);
+    double kp = mean(s_kp);
+    if (kp < 2.0) kp = 2.0;
+    out[(size_t)P_UTHRESH * N + k] = mean(s_hl1);
+    out[(size_t)P_ALPHA * N + k] = mean(s_alpha);
+    out[(size_t)P_KP * N + k] = kp;
+    out[(size_t)P_FASP * N + k] = asp_on ? mean(s_asp) : 0.0;
+    out[(size_t)P_HARSAM * N + k] = (a.proc_pet == 1) ? pp[3] : 0.0;
+}
+
+// One LAI entry's means into their planes (a gridded series:
+// [member][lai_groups][n_lai][N])
+__device__ void put_lai(const MprArgs &a, int m, int mo, int k, double v_int, double v_pet, double v_pet2, double *out)
+{
+    const size_t N = a.n1;
+    if (a.lai_out) {
+        const int ng = lai_groups(a.proc_pet), n_lai = a.n_lai_steps;
+        double *lo = a.lai_out + (size_t)m * ng * n_lai * N + (size_t)mo * N + k;
+        lo[0] = v_int;
+        if (ng > 1) lo[(size_t)n_lai * N] = v_pet;
+        if (ng > 2) lo[(size_t)2 * n_lai * N] = v_pet2;
+    } else {
+        out[(size_t)(P_MAXINTER + mo) * N + k] = v_int;
+        out[(size_t)(P_PETLAI + mo) * N + k] = v_pet;
+        out[(size_t)(P_PET2 + mo) * N + k] = v_pet2;
+    }
+}
+
+// LAI entries part, part + n_parts, ... of a cell: canopy_intercept_param
+// (src/MPR/mo_multi_param_reg.f90:1132-1152) and pet_correctbyLAI, per LAI
+// entry (12 monthly slots or a gridded series: the reference loops over
+// size(LAI0, 2), :1142)
+template <int PET>
+__device__ void upscale_lai(const MprArgs &a, const double *g, int part, int n_parts, int k, int m, int ns, double *out)
+{
+    const size_t N = a.n1, slots = (size_t)a.max_sub * N;
+    const double *pp = g + a.off.pet, gi = g[a.off.interc];
     const double *plai = a.petlai + (size_t)m * 3 * a.n_lai_classes * 12;
     const int n_lai = a.n_lai_steps;
-    for (int mo = 0; mo < n_lai; ++mo) {
-        double s_int = 0.0, s_pet = 0.0, s_pt = 0.0, s_ra = 0.0, s_rs = 0.0;
+    const Mean mean((double)ns);
+    for (int mo = part; mo < n_lai; mo += n_parts) {
+        double s_int = 0.0, s_pet = 0.0, s_pet2 = 0.0;
         for (int j = 0; j < ns; ++j) {
-            const uint32_t c = __ldg(code + (size_t)j * N);
+            const uint32_t c = __ldg(a.code + k + (size_t)j * N);
             if (!a.lai && !bc_ok(BC_MPR_LAI, (c >> 16) & 0xFFu, a.n_lai_classes)) continue;
-            double lai;
-            if (a.lai) {
-                lai = __ldg(a.lai + mo * slots + (size_t)j * N + k);
-            } else {
-                lai = __ldg(a.lai_lut + ((c >> 16) & 0xFFu) * 12 + mo);
-            }
+            const double lai = a.lai ? __ldg(a.lai + mo * slots + (size_t)j * N + k)
+                                     : __ldg(a.lai_lut + ((c >> 16) & 0xFFu) * 12 + mo);
+            const int l = (int)((c & kMprKeyMask) % 3u); // 0 forest, 1 impervious, 2 pervious
             s_int = s_int + lai * gi;
             // priestley_taylor_alpha, src/MPR/mo_mpr_pet.f90:311-369: alpha0 = p1 + p2 LAI0
-            if (a.proc_pet == 2) s_pt = s_pt + (pp[0] + pp[1] * lai);
-            if (a.proc_pet == 3) {
+            if constexpr (PET == 2) s_pet = s_pet + (pp[0] + pp[1] * lai);
+            if constexpr (PET == 3) {
                 // aerodynamical_resistance, src/MPR/mo_multi_param_reg.f90:1165-1262: canopy
                 // height by land cover (pervious: p3 LAI / max over the months), measurement
                 // height 10 m raised above the canopy, log profile with karman = 0.41
-                const int l = (int)((c & kMprKeyMask) % 3u); // 0 forest, 1 impervious, 2 pervious
                 double hc = (l == 0) ? pp[0] : pp[1];
                 if (l == 2) {
                     double mx = -1.0e300;
@@ -362,13 +407,12 @@ __global__ void __launch_bounds__(128) mpr_upscale_kernel(MprArgs a)
                 double zm = 10.0;
                 if (zm < hc) zm = hc + zm;
                 const double disp = pp[3] * hc, z0m = pp[4] * hc, z0h = pp[5] * z0m;
-                s_ra = s_ra + hm_log((zm - disp) / z0m) * hm_log((zm - disp) / z0h) / (0.41 * 0.41);
+                s_pet = s_pet + hm_log((zm - disp) / z0m) * hm_log((zm - disp) / z0h) / (0.41 * 0.41);
                 // bulksurface_resistance, src/MPR/mo_mpr_pet.f90:407-475, capped at 250 s m-1
                 const double rs = pp[6] / (lai / (0.3 * lai + 1.2));
-                s_rs = s_rs + (rs > 250.0 ? 250.0 : rs);
+                s_pet2 = s_pet2 + (rs > 250.0 ? 250.0 : rs);
             }
-            if (a.proc_pet == -1) {
-                const int l = (int)((c & kMprKeyMask) % 3u);
+            if constexpr (PET == -1) {
                 double inv;
                 if (a.lai) {
                     const double base = (l == 0) ? pp[0] : (l == 1) ? pp[1] : pp[2];
@@ -379,22 +423,86 @@ __global__ void __launch_bounds__(128) mpr_upscale_kernel(MprArgs a)
                 s_pet = s_pet + inv;
             }
         }
-        const double v_int = s_int / dn;
-        const double v_pet = (a.proc_pet == -1) ? dn / s_pet
-                             : (a.proc_pet == 2) ? s_pt / dn
-                             : (a.proc_pet == 3) ? s_ra / dn : 0.0;
-        const double v_pet2 = (a.proc_pet == 3) ? s_rs / dn : 0.0;
-        if (a.lai_out) { // a gridded LAI series: [member][lai_groups][n_lai][N]
-            const int ng = lai_groups(a.proc_pet);
-            double *lo = a.lai_out + (size_t)m * ng * n_lai * N + (size_t)mo * N + k;
-            lo[0] = v_int;
-            if (ng > 1) lo[(size_t)n_lai * N] = v_pet;
-            if (ng > 2) lo[(size_t)2 * n_lai * N] = v_pet2;
-        } else {
-            out[(size_t)(P_MAXINTER + mo) * N + k] = v_int;
-            out[(size_t)(P_PETLAI + mo) * N + k] = v_pet;
-            out[(size_t)(P_PET2 + mo) * N + k] = v_pet2;
+        put_lai(a, m, mo, k, mean(s_int), PET == -1 ? hm_div(mean.dn, s_pet) : PET >= 2 ? mean(s_pet) : 0.0,
+                PET == 3 ? mean(s_pet2) : 0.0, out);
+    }
+}
+
+// The same for the 12 months of class LAI where only canopy interception and
+// the LAI correction depend on it: `lg`, the classes' LAI times the canopy
+// factor, was multiplied once for the block
+constexpr int kLaiParts = 2, kPartMonths = 12 / kLaiParts;
+template <int PET>
+__device__ void upscale_lai_classes(const MprArgs &a, const double *lg, int part, int k, int m, int ns, double *out)
+{
+    const size_t N = a.n1;
+    const double *plai = a.petlai + (size_t)m * 3 * a.n_lai_classes * 12;
+    const int mo0 = part * kPartMonths;
+    double s_int[kPartMonths] = {}, s_pet[kPartMonths] = {};
+    for (int j = 0; j < ns; ++j) {
+        const uint32_t c = __ldg(a.code + k + (size_t)j * N), cls = (c >> 16) & 0xFFu;
+        if (!bc_ok(BC_MPR_LAI, cls, a.n_lai_classes)) continue;
+#pragma unroll
+        for (int i = 0; i < kPartMonths; ++i) s_int[i] = s_int[i] + lg[cls * 12 + mo0 + i];
+        if constexpr (PET == -1) {
+            const double *p = plai + ((size_t)((c & kMprKeyMask) % 3u) * a.n_lai_classes + cls) * 12 + mo0;
+#pragma unroll
+            for (int i = 0; i < kPartMonths; ++i) s_pet[i] = s_pet[i] + __ldg(p + i);
         }
+    }
+    const Mean mean((double)ns);
+#pragma unroll
+    for (int i = 0; i < kPartMonths; ++i)
+        put_lai(a, m, mo0 + i, k, mean(s_int[i]), PET == -1 ? hm_div(mean.dn, s_pet[i]) : 0.0, 0.0, out);
+}
+
+// grid (ceil(n1 / 32), members), block 32 cells x (H + 4) warps: a warp per
+// soil horizon, two for the other means, two for the LAI entries.
+//
+// What bounds it: the FP64 pipe (19 cycles of an SM an instruction), so sums
+// of table entries are all that is left on it -- about 40 additions a sub-cell
+// with 3 horizons; divisions run on the integer pipe, and what belongs to
+// another PET process or repeats over the cells is not issued.  One thread a
+// cell issued 143 a sub-cell: 64 members of 9,216 cells with 16 sub-cells each
+// 2.55 ms, 0.98 ms here.  The warps of a cell also shorten its chain where a
+// launch has few cells: mhm_mpr of one member with 9,216 cells 0.24 -> 0.10 ms.
+__global__ void __launch_bounds__(32 * (kMaxHorizons + 4)) mpr_upscale_kernel(MprArgs a)
+{
+    extern __shared__ double s_mpr[]; // [H][32] root fractions, then the classes' LAI times the canopy factor
+    const int lane = threadIdx.x % 32, part = threadIdx.x / 32, H = a.H;
+    const int k = blockIdx.x * 32 + lane, m = blockIdx.y;
+    const double *g = a.gamma + (size_t)m * a.n_gamma;
+    const double *tab = a.table + (size_t)m * a.n_keys * mpr_table_stride(H);
+    double *out = a.params + (size_t)m * a.member_stride;
+    double *lg = s_mpr + H * 32;
+    const bool here = k < a.n1;
+    const int ns = here ? a.nsub[k] : 0;
+    if (!a.lai)
+        for (int i = threadIdx.x; i < a.n_lai_classes * 12; i += blockDim.x) lg[i] = a.lai_lut[i] * g[a.off.interc];
+    double froots = 0.0;
+    if (here && part < H) froots = upscale_horizon(a, part, k, ns, tab, out);
+    if (part < H) s_mpr[part * 32 + lane] = froots;
+    __syncthreads();
+    if (!here) return;
+    if (part < H) { // the root normalisation of mpr_SMhorizons
+        double ftot = 0.0;
+        for (int h = 0; h < H; ++h) {
+            const double f = s_mpr[h * 32 + lane];
+            if (f > 0.0) ftot = ftot + f;
+        }
+        out[(size_t)(P_HORIZON + part) * a.n1 + k] = (ftot > 0.0) ? hm_div(froots, ftot) : 0.0;
+    } else if (part == H) {
+        upscale_recession(a, g, k, ns, tab, out);
+    } else if (part == H + 1) {
+        upscale_aspect(a, g, k, ns, tab, out);
+    } else {
+        const int p = part - H - 2;
+        if (a.proc_pet == 2) upscale_lai<2>(a, g, p, kLaiParts, k, m, ns, out);
+        else if (a.proc_pet == 3) upscale_lai<3>(a, g, p, kLaiParts, k, m, ns, out);
+        else if (a.proc_pet == -1 && !a.lai) upscale_lai_classes<-1>(a, lg, p, k, m, ns, out);
+        else if (a.proc_pet == -1) upscale_lai<-1>(a, g, p, kLaiParts, k, m, ns, out);
+        else if (!a.lai) upscale_lai_classes<0>(a, lg, p, k, m, ns, out);
+        else upscale_lai<0>(a, g, p, kLaiParts, k, m, ns, out);
     }
 }
 
@@ -403,11 +511,13 @@ __global__ void __launch_bounds__(128) mpr_upscale_kernel(MprArgs a)
 cudaError_t launch_mpr(const MprArgs &a, cudaStream_t s)
 {
     if (a.n_members <= 0) return cudaSuccess;
-    const int rows = a.n_keys + ((a.proc_pet == -1) ? 3 * a.n_lai_classes * 12 : 0);
-    mpr_table_kernel<<<dim3((rows + 63) / 64, a.n_members), 64, 0, s>>>(a);
+    const int row_blocks = (a.n_keys + kTableRows - 1) / kTableRows, bs = kTableRows * kRowLanes;
+    const int lai_blocks = a.proc_pet == -1 ? (3 * a.n_lai_classes * 12 + bs - 1) / bs : 0;
+    mpr_table_kernel<<<dim3(row_blocks + lai_blocks, a.n_members), bs, 0, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    mpr_upscale_kernel<<<dim3((a.n1 + 127) / 128, a.n_members), 128, 0, s>>>(a);
+    const size_t smem = ((size_t)a.H * 32 + (a.lai ? 0 : (size_t)a.n_lai_classes * 12)) * sizeof(double);
+    mpr_upscale_kernel<<<dim3((a.n1 + 31) / 32, a.n_members), 32 * (a.H + 4), smem, s>>>(a);
     return cudaGetLastError();
 }
 

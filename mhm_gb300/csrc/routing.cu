@@ -437,14 +437,17 @@ __global__ void gauge_gather_kernel(const GaugeArgs a)
     a.q_gauge[((size_t)m * a.n_gauges + g) * a.total_steps + a.step_offset + t] = v;
 }
 
-// reg_rout, src/mRM/mo_mrm_mpr.f90:61-119, one thread per link; ss_max is the
-// basin's max slope (parameter independent, computed on the host once).
-__global__ void reg_rout_kernel(int n_links, const double *p5, double ss_max, double TS,
+// reg_rout, src/mRM/mo_mrm_mpr.f90:61-119, one thread per link and member (the
+// grid's second dimension; its parameters p5_stride after the previous one's);
+// ss_max is the basin's max slope (parameter independent, computed on the host
+// once).
+__global__ void reg_rout_kernel(int n_links, int n_nodes, const double *p5, int p5_stride, double ss_max, double TS,
                                 const double *length, const double *slope, const double *ffp,
                                 const int32_t *link_pos, double *C1, double *C2)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_links) return;
+    p5 += (size_t)blockIdx.y * p5_stride;
     const double p0 = p5[0], p1 = p5[1], p2 = p5[2], p3 = p5[3], p4 = p5[4];
     double K = p0 + p1 * (length[i] * 0.001) + p2 * slope[i] + p3 * ffp[i];
     double xi = p4 * (1.0 + slope[i] / ss_max);
@@ -453,7 +456,7 @@ __global__ void reg_rout_kernel(int n_links, const double *p5, double ss_max, do
     if (K > 0.5 * TS / xi) K = 0.5 * TS / xi;
     if (K < 0.5 * TS / (1.0 - xi)) K = 0.5 * TS / (1.0 - xi);
     const double c1 = TS / (K * (1.0 - xi) + 0.5 * TS);
-    const int pos = link_pos[i];
+    const size_t pos = (size_t)blockIdx.y * n_nodes + link_pos[i];
     C1[pos] = c1;
     C2[pos] = 1.0 - c1 * K / TS;
 }
@@ -501,13 +504,13 @@ cudaError_t launch_gauge_gather(const GaugeArgs &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_reg_rout(int n_links, const double *p5, double ss_max, double TS, const double *length,
-                            const double *slope, const double *ffp, const int32_t *link_pos, double *C1,
-                            double *C2, cudaStream_t s)
+cudaError_t launch_reg_rout(int n_members, int n_links, int n_nodes, const double *p5, int p5_stride, double ss_max,
+                            double TS, const double *length, const double *slope, const double *ffp,
+                            const int32_t *link_pos, double *C1, double *C2, cudaStream_t s)
 {
-    if (n_links <= 0) return cudaSuccess;
-    reg_rout_kernel<<<(n_links + 127) / 128, 128, 0, s>>>(n_links, p5, ss_max, TS, length, slope, ffp, link_pos,
-                                                          C1, C2);
+    if (n_links <= 0 || n_members <= 0) return cudaSuccess;
+    reg_rout_kernel<<<dim3((n_links + 127) / 128, n_members), 128, 0, s>>>(n_links, n_nodes, p5, p5_stride, ss_max, TS,
+                                                                           length, slope, ffp, link_pos, C1, C2);
     return cudaGetLastError();
 }
 
