@@ -33,6 +33,7 @@ cudaError_t launch_route_flow(const RouteArgs &a, int round, cudaStream_t s);
 cudaError_t launch_qmod_step(const QmodStepArgs &a, cudaStream_t s);
 cudaError_t launch_gauge_gather(const GaugeArgs &a, cudaStream_t s);
 cudaError_t launch_qrouted(const QroutArgs &a, cudaStream_t s);
+cudaError_t launch_init_states(const InitArgs &a, cudaStream_t s);
 cudaError_t launch_reg_rout(int n_members, int n_links, int n_nodes, const double *p5, int p5_stride, double ss_max,
                             double TS, const double *length, const double *slope, const double *ffp,
                             const int32_t *link_pos, double *C1, double *C2, cudaStream_t s);
@@ -1087,27 +1088,26 @@ int mhm_init_states(mhm_ctx *ctx, int32_t m, const double *hd)
     ON_CTX_DEVICE(ctx);
     if (int rc = mhm_sync(ctx)) return rc; // no enqueued step may still read what changes
     if (m < 0 || m >= ctx->M) return fail(ctx, MHM_ERR_INVALID, "member out of range");
-    const size_t N = ctx->N;
-    const int H = ctx->H, ns = n_state_planes(H);
+    const size_t L = ctx->L;
+    const int H = ctx->H;
+    InitArgs a{};
+    a.n_cells = ctx->N;
+    a.n_planes = n_state_planes(H);
+    a.states = ctx->states.p + (size_t)m * a.n_planes * ctx->N;
     // mo_init_states.f90:258-345: interc 0, snow 15, sealed 0, unsat 10, sat 75,
     // SM(h) = (depth(h) - depth(h-1)) * 0.25, last horizon to 1500 mm
-    std::vector<double> s((size_t)ns * N);
-    auto plane = [&](int pl, double v) { std::fill(s.begin() + (size_t)pl * N, s.begin() + (size_t)(pl + 1) * N, v); };
-    plane(S_INTERC, 0.0);
-    plane(S_SNOW, 15.0);
-    plane(S_SEAL, 0.0);
-    plane(S_UNSAT, 10.0);
-    plane(S_SAT, 75.0);
-    for (int h = 0; h < H - 1; ++h) plane(S_SM + h, (h == 0 ? hd[0] : hd[h] - hd[h - 1]) * 0.25);
-    plane(S_SM + H - 1, (1500.0 - (H >= 2 ? hd[H - 2] : 0.0)) * 0.25);
-    CK(cudaMemcpyAsync(ctx->states.p + (size_t)m * ns * N, s.data(), s.size() * sizeof(double),
-                       cudaMemcpyHostToDevice, ctx->stream),
-       "states");
+    a.value[S_SNOW] = 15.0;
+    a.value[S_UNSAT] = 10.0;
+    a.value[S_SAT] = 75.0;
+    for (int h = 0; h < H - 1; ++h) a.value[S_SM + h] = (h == 0 ? hd[0] : hd[h] - hd[h - 1]) * 0.25;
+    a.value[S_SM + H - 1] = (1500.0 - (H >= 2 ? hd[H - 2] : 0.0)) * 0.25;
     if (ctx->proc_rout >= 1) {
-        const size_t L = ctx->L;
-        for (auto *b : {&ctx->qtin1, &ctx->qtr1, &ctx->qout_last, &ctx->qmod_last})
-            CK(cudaMemsetAsync(b->p + m * L, 0, L * sizeof(double), ctx->stream), "routing states");
+        a.n_nodes = ctx->L;
+        int r = 0;
+        for (auto *b : {&ctx->qtin1, &ctx->qtr1, &ctx->qout_last, &ctx->qmod_last}) a.routing[r++] = b->p + m * L;
     }
+    CK(launch_init_states(a, ctx->stream), "states");
+    g_launches++;
     CK(cudaStreamSynchronize(ctx->stream), "states sync");
     return MHM_OK;
 }

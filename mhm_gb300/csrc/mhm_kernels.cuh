@@ -274,6 +274,14 @@ struct GaugeArgs {
     const int32_t *member_step0; // member mode: idle members get zero discharge
 };
 
+// initial states of one member
+struct InitArgs {
+    int32_t n_cells, n_nodes, n_planes;  // n_nodes = 0: no routing states
+    double value[S_SM + kMaxHorizons];   // by state plane
+    double *states;                      // [n_planes][n_cells]
+    double *routing[4];                  // [n_nodes] each
+};
+
 // ---- multiscale parameter regionalisation ----
 constexpr int kMprMaxSoilHor = 16;
 // entries of one (soil, land cover) row of the per-member soil table
