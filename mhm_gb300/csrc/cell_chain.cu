@@ -92,9 +92,13 @@ cudaError_t launch_cell_chain_fused(const FusedCellArgs &f, int hl, bool lean, i
 cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
 {
     if (H < 1 || H > kMaxHorizons) return cudaErrorInvalidValue;
-    // per-step fluxes or aggregated outputs: one variant
-    if (a.flux_aet || a.out.n_planes > 0) return launch_cell_chain_variant<4, true>(a, H, s);
+    // per-step fluxes or aggregated outputs: one register variant.  With 3 blocks
+    // an SM they hold what a step adds up; with 4 some of it goes through local
+    // memory, with 2 a large launch lacks warps (3 horizons, 14 planes, 240 steps,
+    // 4 / 3 / 2 blocks: 3,600 cells 2.76 / 2.56 / 2.50 ms, 40,000 cells 3.62 /
+    // 3.40 / 5.69, 160,000 cells 11.9 / 10.3 / 14.3).
     if (cell_chain_fits_small(a)) return launch_cell_chain_small(a, s);
+    if (a.flux_aet || a.out.n_planes > 0) return launch_cell_chain_variant<3, true>(a, H, s);
     switch (occ) {
     case 6: return launch_cell_chain_o6(a, H, s);
     case 8: return launch_cell_chain_o8(a, H, s);

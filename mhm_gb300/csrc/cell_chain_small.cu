@@ -33,12 +33,20 @@ __device__ __forceinline__ void bar_sync(int id, int threads)
 // forcing 14.6 -> 5.0 ms.
 //
 // 64 registers a thread, so that as many blocks as possible are resident.
-template <int H, bool LEAN>
-__global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chain_small_kernel(const CellArgs a)
+//
+// FLUX, aggregated outputs or per-step fluxes: one more warp adds up what the
+// others post of a step while they work on the next.
+template <int H, bool LEAN, bool FLUX>
+__global__ void __launch_bounds__(32 * (H + 2 + FLUX), 1024 / (32 * (H + 2 + FLUX)))
+    cell_chain_small_kernel(const CellArgs a)
 {
     __shared__ double s_sm[H][32], s_fr[H][32], s_st[H][32], s_sms[H][32];
     __shared__ double s_pe[2][32], s_demand[2][32], s_rsealed[2][32]; // by parity of the step
-    constexpr int n_warps = H + 2;
+    // posted for the outputs, by step: the surface's values (the surface is two
+    // steps ahead of the reader), the values below
+    constexpr int kSurf = 9, kBelow = 7, kPost = FLUX ? 32 : 1;
+    __shared__ double s_surf[3][kSurf][kPost], s_below[2][kBelow][kPost], s_out[2][3][H][kPost]; // SM, aET, infiltration
+    constexpr int n_warps = H + 2 + FLUX;
     const int lane = threadIdx.x & 31;
     // parts start at another warp in each block of an SM, so that the
     // schedulers share them
@@ -67,7 +75,7 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
     double *S = a.states + (size_t)m * n_state_planes(H) * N + k;
     auto par = [&](int plane) { return __ldg(P + (size_t)plane * N); };
     const bool feddes = LEAN || (a.proc_sm == 1 || a.proc_sm == 4);
-    constexpr int all = 32 * n_warps, below = all - 32; // below: without the surface
+    constexpr int all = 32 * n_warps, below = 32 * (H + 1); // below: the soil and the horizons
     constexpr uint64_t kExpOne = 0x0010000000000000ull; // as in cell_chain_item
     uint64_t nonfin = 0;
     auto chk = [&](double x) { nonfin |= hm_abs_bits(hm_d2b(x)) + kExpOne; };
@@ -87,9 +95,16 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
                 s_pe[t & 1][lane] = sf.prec_effect;
                 s_demand[t & 1][lane] = sf.pet - sf.aet_can;
                 s_rsealed[t & 1][lane] = sf.runoff_sealed;
+                if constexpr (FLUX) {
+                    const double v[kSurf] = {sf.interc, sf.snow, sf.seal, sf.pet, sf.aet_can, sf.aet_sealed_act,
+                                             sf.runoff_sealed, sf.prec_effect, sf.melt};
+#pragma unroll
+                    for (int i = 0; i < kSurf; ++i) s_surf[t % 3][i][lane] = v[i];
+                }
             }
             bar_sync(1, all); // step t above the soil; the soil has taken step t - 1 from the other buffer
         }
+        if (FLUX) bar_sync(1, all);
         if (active) {
             S[(size_t)S_INTERC * N] = sf.interc;
             S[(size_t)S_SNOW * N] = sf.snow;
@@ -133,7 +148,11 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
                                 s_sm[h][lane] = filled;
                             }
                         }
+                        if constexpr (FLUX) s_out[t & 1][2][h][lane] = infil;
                     }
+                } else if constexpr (FLUX) {
+#pragma unroll
+                    for (int h = 0; h < H; ++h) s_out[t & 1][2][h][lane] = 0.0;
                 }
             }
             bar_sync(2, below); // the soil moisture after infiltration
@@ -155,6 +174,7 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
                     double left = hm_sel(enough, d, kEps);
                     left = hm_sel(hm_lt(left, kEps), kEps, left);
                     s_sm[h][lane] = left;
+                    if constexpr (FLUX) s_out[t & 1][0][h][lane] = left, s_out[t & 1][1][h][lane] = aet;
                     if (h == 0) {
                         aet_above = hm_sel(hm_gt0(aet), aet, 0.0);
                     } else if (h + 1 < H) {
@@ -168,14 +188,73 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
                 const double q_total = gd.total(fnotsealed, s_rsealed[t & 1][lane], fsealed);
                 tro[(size_t)t * out_stride] = q_total;
                 chk(q_total);
+                if constexpr (FLUX) {
+                    const double v[kBelow] = {gd.unsat, gd.sat, gd.fast, gd.slow, gd.base, gd.perc, q_total};
+#pragma unroll
+                    for (int i = 0; i < kBelow; ++i) s_below[t & 1][i][lane] = v[i];
+                }
             }
         }
+        if (FLUX) bar_sync(1, all);
         if (active) {
             S[(size_t)S_UNSAT * N] = gd.unsat;
             S[(size_t)S_SAT * N] = gd.sat;
             chk(gd.unsat);
             chk(gd.sat);
         }
+    } else if (FLUX && part == H + 2) { // outputs
+        extern __shared__ double s_acc[]; // the running sums, [plane][32]
+        const OutArgs &o = a.out;
+        const size_t at = (size_t)m * N + k;
+        const double fsealed = par(P_FSEALED), fnotsealed = 1.0 - fsealed, karst = par(P_KARST);
+        double osat = 0.0;
+        for (int h = 0; h < H; ++h) osat = osat + par(P_HORIZON + H + h);
+        const uint64_t r_osat = hm_recip_of(osat);
+        int cnt = o.cnt0, slot = o.slot0;
+        const int64_t tt_w = o.n_planes > 0 && o.tt_w ? o.tt_w[m] : -1;
+        if (active)
+            for (int v = 0; v < o.n_planes; ++v) s_acc[v * 32 + lane] = o.acc[(size_t)v * out_stride + at];
+        auto add = [&](int plane, double x) { s_acc[plane * 32 + lane] = s_acc[plane * 32 + lane] + x; };
+        bar_sync(1, all);
+        for (int t = 0; t < a.n_steps; ++t) {
+            bar_sync(1, all); // step t below the soil, step t + 1 above it
+            if (active) {
+                const auto &u = s_surf[t % 3];
+                const auto &d = s_below[t & 1];
+                const auto &q = s_out[t & 1];
+                double aet_soil = 0.0;
+#pragma unroll
+                for (int h = 0; h < H; ++h) aet_soil = aet_soil + q[1][h][lane];
+                const OutStep v{u[0][lane], u[1][lane], u[2][lane], u[3][lane], u[4][lane], u[5][lane],
+                                u[6][lane], u[7][lane], u[8][lane], d[0][lane], d[1][lane], d[2][lane],
+                                d[3][lane], d[4][lane], d[5][lane], d[6][lane], aet_soil};
+                if (a.flux_aet) {
+                    const size_t fo = (size_t)t * out_stride + at;
+                    a.flux_aet[fo] = v.aet_can + fsealed * v.aet_sealed + fnotsealed * aet_soil;
+                    a.flux_loss[fo] = fnotsealed * (v.perc - v.perc * karst);
+                }
+                const int64_t tt = o.tt_base + t;
+                if (o.n_planes > 0 && tt > o.warm_steps) {
+                    // the weights of cell_chain_item
+                    const bool ow = tt == tt_w;
+                    double ofs = fsealed, ofns = fnotsealed;
+                    if (ow) {
+                        ofs = o.w_fsealed[at];
+                        ofns = 1.0 - ofs;
+                    }
+                    for (int h = 0; h < H; ++h) {
+                        if (o.plane[OF_INFIL] >= 0) add(o.plane[OF_INFIL] + h, q[2][h][lane] * ofns);
+                        if (o.plane[OF_AET_L] >= 0) add(o.plane[OF_AET_L] + h, q[1][h][lane] * ofns);
+                    }
+                    out_add(
+                        o, H, v, ow, ofs, ofns, osat, r_osat, add, [&](int h) { return q[0][h][lane]; },
+                        [&](int h) { return ow ? o.w_sms[((size_t)m * H + h) * N + k] : par(P_HORIZON + H + h); });
+                    out_close(o, s_acc + lane, 32, out_stride, at, tt, steps[t].dflags, cnt, slot);
+                }
+            }
+        }
+        if (active)
+            for (int v = 0; v < o.n_planes; ++v) o.acc[(size_t)v * out_stride + at] = s_acc[v * 32 + lane];
     } else { // horizon h
         const int h = part - 2;
         const double froots = par(P_HORIZON + h), sms = par(P_HORIZON + H + h), fc = par(P_HORIZON + 2 * H + h),
@@ -197,6 +276,7 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
             bar_sync(2, below);
             bar_sync(2, below);
         }
+        if (FLUX) bar_sync(1, all);
         if (active) {
             const double smh = s_sm[h][lane];
             S[(size_t)(S_SM + h) * N] = smh;
@@ -208,14 +288,15 @@ __global__ void __launch_bounds__(32 * (H + 2), 1024 / (32 * (H + 2))) cell_chai
 
 } // namespace
 
-template <bool LEAN> static cudaError_t launch_small(const CellArgs &a, cudaStream_t s)
+template <bool LEAN, bool FLUX> static cudaError_t launch_small(const CellArgs &a, cudaStream_t s)
 {
+    const size_t smem = FLUX ? (size_t)a.out.n_planes * 32 * sizeof(double) : 0;
     const int64_t n = (int64_t)a.n_cells * a.n_members;
     const unsigned grid = (unsigned)((n + 31) / 32);
     switch (a.n_horizons) {
 #define MHM_CASE(HH)                                                                                               \
     case HH:                                                                                                       \
-        cell_chain_small_kernel<HH, LEAN><<<grid, 32 * (HH + 2), 0, s>>>(a);                                       \
+        cell_chain_small_kernel<HH, LEAN, FLUX><<<grid, 32 * (HH + 2 + FLUX), smem, s>>>(a);                                     \
         return cudaGetLastError();
         MHM_CASE(1) MHM_CASE(2) MHM_CASE(3) MHM_CASE(4) MHM_CASE(5) MHM_CASE(6) MHM_CASE(7) MHM_CASE(8)
 #undef MHM_CASE
@@ -228,15 +309,22 @@ template <bool LEAN> static cudaError_t launch_small(const CellArgs &a, cudaStre
 // the GPU at once (96 steps, this kernel / one thread a cell: 1 horizon, 40,000
 // cells 0.45 / 0.67 ms, 62,500 cells 0.80 / 0.76; 3 horizons, 25,600 cells 0.51 /
 // 0.78, 40,000 cells 0.81 / 0.88, 62,500 cells 1.25 / 0.99; 6 horizons, 16,384
-// cells 0.61 / 0.96, 25,600 cells 1.01 / 1.10, 40,000 cells 1.48 / 1.25).
+// cells 0.61 / 0.96, 25,600 cells 1.01 / 1.10, 40,000 cells 1.48 / 1.25).  With
+// outputs, whose warp takes more off the other kernel's chain, up to 235,000
+// (cells times H + 3; 14 or more planes: 1 horizon, 3,600 cells 0.27 / 0.72,
+// 62,500 cells 1.20 / 1.91; 3 horizons, 3,600 cells 0.38 / 0.95, 25,600 cells
+// 1.00 / 1.14, 40,000 cells 1.31 / 1.31, 52,900 cells 1.75 / 1.34; 6 horizons,
+// 9,216 cells 0.68 / 1.35, 25,600 cells 1.33 / 1.59, 40,000 cells 1.98 / 1.83).
 bool cell_chain_fits_small(const CellArgs &a)
 {
-    return a.small_ok && (int64_t)a.n_cells * a.n_members * (a.n_horizons + 2) <= 180000;
+    const bool flux = a.flux_aet || a.out.n_planes > 0;
+    return a.small_ok && (int64_t)a.n_cells * a.n_members * (a.n_horizons + 2 + flux) <= (flux ? 235000 : 180000);
 }
 
 cudaError_t launch_cell_chain_small(const CellArgs &a, cudaStream_t s)
 {
-    return cell_chain_lean(a) ? launch_small<true>(a, s) : launch_small<false>(a, s);
+    if (a.flux_aet || a.out.n_planes > 0) return launch_small<false, true>(a, s);
+    return cell_chain_lean(a) ? launch_small<true, false>(a, s) : launch_small<false, false>(a, s);
 }
 
 } // namespace mhm

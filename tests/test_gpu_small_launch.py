@@ -113,3 +113,42 @@ def test_members_at_their_own_steps(monkeypatch):
     for a, b in zip(out[0][1], out[1][1]):
         for k in STATES:
             assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("flags", ["all", "few"])
+@pytest.mark.parametrize("H,nr,nc,pet,sm,hourly,members", [
+    (1, 1, 1, 0, 1, True, 1), (2, 4, 8, 0, 4, True, 2), (3, 3, 11, 0, 1, False, 1), (6, 7, 9, 1, 3, False, 3),
+    (8, 9, 9, 0, 2, True, 2)])
+def test_outputs_small_equals_one_thread_a_cell(monkeypatch, flags, H, nr, nc, pet, sm, hourly, members):
+    """The running sums of the output warp, and those the other kernel keeps in
+    shared memory (few planes) or in device memory (all, 8 horizons): every
+    output variable over daily intervals cut by calls and chunks, a warm-up,
+    a step with its own weights, and the per-step fluxes."""
+    from mhm_gb300.model import MhmGpu
+    dom = synth.make_domain(nr, nc, H, l11_factor=2, seed=3)
+    ps = [_params(dom, pet, 20 + m) for m in range(members)]
+    f = _forcing(dom, pet, hourly, 80 if hourly else 4)
+    rng = np.random.default_rng(2)
+    w_fs, w_sms = rng.uniform(0.0, 0.5, dom.n_cells), rng.uniform(100.0, 300.0, (H, dom.n_cells))
+    res = []
+    for small in (1, 0):
+        monkeypatch.setenv("MHM_CELL_SMALL", str(small))
+        monkeypatch.setenv("MHM_CHUNK_BYTES", str(2 * members * dom.n_cells * 8 * 30))
+        g = MhmGpu(dom, proc_soilmoist=sm, proc_pet=pet, hourly=hourly, n_members=members)
+        try:
+            g.prepare(ps, synth.ROUTING_PARAMS_DEFAULT)
+            g.set_meteo(1, **f)
+            g.enable_flux_state_outputs([i for i in range(1, 22) if i != 18] if flags == "all" else (3, 9, 10, 21), -1, 5, 10**9, max_slots=5)
+            g.enable_fluxes()
+            g.set_output_weights(members - 1, 40, w_fs, w_sms)
+            q = [g.run(1, 31)]
+            fx = list(g.get_fluxes())
+            q.append(g.run(32, 49))
+            fx += g.get_fluxes()
+            names, fs, at = g.read_flux_state_outputs()
+            res.append(q + fx + [fs, at] + [g.get_state(m)[k] for m in range(members) for k in STATES])
+        finally:
+            g.close()
+    assert res[0][6].shape[0] == 3 and np.isfinite(res[0][6]).all() and np.any(res[0][6] != 0.0)
+    for i, (a, b) in enumerate(zip(*res)):
+        assert np.array_equal(a, b), i
