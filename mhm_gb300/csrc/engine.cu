@@ -101,6 +101,8 @@ struct OutSet {
     DevBuf<double> acc, out;
 };
 
+constexpr int kMaxPieces = 10; // a chunk's host forcing arrives in up to so many
+
 struct ForcingSrc {
     const double *ptr = nullptr;
     int32_t row0 = 0, n_rows = 0, on_device = 0;
@@ -179,7 +181,7 @@ struct mhm_ctx {
     int32_t last_steps = 0;
     // execution
     cudaStream_t stream = nullptr, copy_stream = nullptr, route_stream = nullptr;
-    cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
+    cudaEvent_t ev_copied[2][kMaxPieces] = {}, ev_consumed[2] = {nullptr, nullptr};
     cudaEvent_t ev_cell_done[2] = {nullptr, nullptr}, ev_acc_done[2] = {nullptr, nullptr};
     cudaEvent_t ev_route_end = nullptr, run_a = nullptr;
     cudaEvent_t ev_poll[3] = {nullptr, nullptr, nullptr};
@@ -662,7 +664,7 @@ int mhm_ctx_create(const mhm_domain_desc *d, int32_t device, mhm_ctx **out)
         return MHM_ERR_CUDA;
     }
     for (int i = 0; i < 2; ++i) {
-        cudaEventCreateWithFlags(&ctx->ev_copied[i], cudaEventDisableTiming);
+        for (cudaEvent_t &e : ctx->ev_copied[i]) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ctx->ev_consumed[i], cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ctx->ev_cell_done[i], cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ctx->ev_acc_done[i], cudaEventDisableTiming);
@@ -764,7 +766,8 @@ int mhm_ctx_destroy(mhm_ctx *ctx)
     if (ctx->route_stream) cudaStreamSynchronize(ctx->route_stream);
     harvest_timing(ctx);
     for (int i = 0; i < 2; ++i) {
-        if (ctx->ev_copied[i]) cudaEventDestroy(ctx->ev_copied[i]);
+        for (cudaEvent_t e : ctx->ev_copied[i])
+            if (e) cudaEventDestroy(e);
         if (ctx->ev_consumed[i]) cudaEventDestroy(ctx->ev_consumed[i]);
         if (ctx->ev_cell_done[i]) cudaEventDestroy(ctx->ev_cell_done[i]);
         if (ctx->ev_acc_done[i]) cudaEventDestroy(ctx->ev_acc_done[i]);
@@ -1335,20 +1338,50 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         r1 = (int32_t)((t1 + stride - 1) / stride);
     };
     const int64_t seq0 = ctx->chunk_seq;
-    auto issue_copy = [&](int c) -> int {
-        if (on_device || c >= nchunks) return MHM_OK;
+    // Host forcing reaches a chunk's staging rows in pieces, and the cell chain of
+    // a piece runs while the next is on its way; accumulation and routing still
+    // take the whole chunk.  Pieces start small, since the first one's copy is
+    // waited for, and grow to a sixth of the chunk: 250,000 cells with 6 horizons,
+    // 240 hourly steps of pinned forcing (1.44 GB) 21.6 ms in one piece, 15.8 so.  Less
+    // than 64 MB goes in one: its copy takes less than the launches it would cost.
+    int32_t n_kinds = 0;
+    for (int k = 0; k < kForcKinds; ++k) n_kinds += need[k];
+    auto piece_ends = [&](int c) { // the chunk's steps in which pieces end
+        const int32_t s0 = c * Tc, nT = std::min(n_steps, s0 + Tc) - s0;
+        std::vector<int32_t> ends;
+        if (!on_device) {
+            int32_t r0, r1;
+            chunk_rows(c, r0, r1);
+            const double rows = r1 - r0 + 1, mb = rows * n_kinds * (double)N * 8e-6;
+            double size = std::max(rows / 24.0, 16.0 * rows / mb);
+            for (double r = size; mb >= 64.0 && r < rows && (int)ends.size() < kMaxPieces - 1; r += size) {
+                // steps of the chunk whose forcing row is among the first r
+                const int32_t e = (int32_t)(((int64_t)r0 + (int64_t)r - 1) * stride - ((int64_t)tt0 + s0) + 1);
+                if (e > (ends.empty() ? 0 : ends.back()) && e < nT) ends.push_back(e);
+                size = std::min(2.0 * size, rows / 6.0);
+            }
+        }
+        ends.push_back(nT);
+        return ends;
+    };
+    // the forcing rows of steps p0 .. p1 - 1 of chunk c, as its piece p
+    auto issue_copy = [&](int c, int p, int32_t p0, int32_t p1) -> int {
         const int slot = (int)((seq0 + c) & 1);
+        const int64_t t0 = (int64_t)tt0 + c * Tc;
         int32_t r0, r1;
         chunk_rows(c, r0, r1);
-        if (ctx->slot_used[slot]) CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_consumed[slot], 0), "wait slot");
+        const int32_t q0 = p == 0 ? r0 : (int32_t)((t0 + p0 - 1 + stride - 1) / stride) + 1; // after the last piece's
+        const int32_t q1 = (int32_t)((t0 + p1 - 1 + stride - 1) / stride);
+        if (p == 0 && ctx->slot_used[slot])
+            CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_consumed[slot], 0), "wait slot");
         for (int k = 0; k < kForcKinds; ++k) {
-            if (!need[k]) continue;
+            if (!need[k] || q1 < q0) continue;
             const ForcingSrc &f = ctx->forc[k];
-            CK(cudaMemcpyAsync(ctx->stage[k][slot].p, f.ptr + (size_t)(r0 - f.row0) * N,
-                               (size_t)(r1 - r0 + 1) * N * sizeof(double), cudaMemcpyHostToDevice, ctx->copy_stream),
+            CK(cudaMemcpyAsync(ctx->stage[k][slot].p + (size_t)(q0 - r0) * N, f.ptr + (size_t)(q0 - f.row0) * N,
+                               (size_t)(q1 - q0 + 1) * N * sizeof(double), cudaMemcpyHostToDevice, ctx->copy_stream),
                "forcing H2D");
         }
-        CK(cudaEventRecord(ctx->ev_copied[slot], ctx->copy_stream), "record copied");
+        CK(cudaEventRecord(ctx->ev_copied[slot][p], ctx->copy_stream), "record copied");
         return MHM_OK;
     };
     if (members) {
@@ -1389,9 +1422,7 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         cudaEventCreate(&ctx->run_a);
         cudaEventRecord(ctx->run_a, ctx->stream);
     }
-    if (int rc = issue_copy(0)) return rc;
     for (int c = 0; c < nchunks; ++c) {
-        if (int rc = issue_copy(c + 1)) return rc;
         const int32_t s0 = c * Tc;
         const int32_t nT = std::min(n_steps, s0 + Tc) - s0;
         const int slot = (int)((seq0 + c) & 1);
@@ -1431,7 +1462,6 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
             a.n_forc_rows = r1 - r0 + 1;
             for (int k = 0; k < kForcKinds; ++k)
                 if (need[k]) fp[k] = ctx->stage[k][slot].p;
-            CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copied[slot], 0), "wait copied");
         }
         a.pre = fp[0];
         a.temp = fp[1];
@@ -1472,36 +1502,54 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
             a.flux_aet = ctx->flux_d[0].p;
             a.flux_loss = ctx->flux_d[1].p;
         }
-        if (ctx->fso.on) {
-            OutArgs &o = a.out;
-            o.n_planes = ctx->fso.n_planes;
-            o.interval = ctx->fso.interval;
-            o.warm_steps = ctx->fso.warm;
-            o.n_tt = ctx->fso.n_tt;
-            o.tt_base = (int64_t)tt0 + s0;
-            o.slot0 = ctx->fso.slots;
-            o.cnt0 = ctx->fso.cnt;
-            o.max_slots = ctx->fso.max_slots;
-            std::memcpy(o.plane, ctx->fs_plane, sizeof(o.plane));
-            o.avg_mask = ctx->fs_avg;
-            o.acc = ctx->fso.acc.p;
-            o.out = ctx->fso.out.p;
-            o.tt_w = ctx->w_tt.p;
-            o.w_fsealed = ctx->w_fs.p;
-            o.w_sms = ctx->w_sms.p;
-            out_advance(ctx->fso, ctx->jul_start, ctx->timestep, (int64_t)tt0 + s0, nT, true);
-        }
         if (fs && fs->phase == 1) {
             fs->args = a; // everything up to the cell chain is enqueued; the rest follows in phase 2
             return MHM_OK;
         }
-        if (fs) {
-            CK(cudaStreamWaitEvent(ctx->stream, fs->ev_fused, 0), "wait fused cell chain");
-        } else {
+        if (fs) CK(cudaStreamWaitEvent(ctx->stream, fs->ev_fused, 0), "wait fused cell chain");
+        const std::vector<int32_t> ends = piece_ends(c);
+        for (int p = 0; !fs && p < (int)ends.size(); ++p) {
+            const int32_t p0 = p == 0 ? 0 : ends[p - 1], p1 = ends[p];
+            if (!on_device) {
+                if (c == 0)
+                    if (int rc = issue_copy(c, p, p0, p1)) return rc;
+                CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copied[slot][p], 0), "wait copied");
+            }
+            CellArgs b = a;
+            b.n_steps = p1 - p0;
+            b.reset_sm = a.reset_sm && p0 == 0;
+            const size_t at = (size_t)p0 * M * N;
+            if (!members) b.steps += p0;
+            b.tro += at;
+            if (a.flux_aet) b.flux_aet += at, b.flux_loss += at;
+            if (ctx->fso.on) {
+                OutArgs &o = b.out;
+                o.n_planes = ctx->fso.n_planes;
+                o.interval = ctx->fso.interval;
+                o.warm_steps = ctx->fso.warm;
+                o.n_tt = ctx->fso.n_tt;
+                o.tt_base = (int64_t)tt0 + s0 + p0;
+                o.slot0 = ctx->fso.slots;
+                o.cnt0 = ctx->fso.cnt;
+                o.max_slots = ctx->fso.max_slots;
+                std::memcpy(o.plane, ctx->fs_plane, sizeof(o.plane));
+                o.avg_mask = ctx->fs_avg;
+                o.acc = ctx->fso.acc.p;
+                o.out = ctx->fso.out.p;
+                o.tt_w = ctx->w_tt.p;
+                o.w_fsealed = ctx->w_fs.p;
+                o.w_sms = ctx->w_sms.p;
+                out_advance(ctx->fso, ctx->jul_start, ctx->timestep, o.tt_base, b.n_steps, true);
+            }
             Bracket br(ctx, 0, ctx->stream);
-            CK(launch_cell_chain(a, H, ctx->cell_occ, ctx->stream), "cell chain launch");
+            CK(launch_cell_chain(b, H, ctx->cell_occ, ctx->stream), "cell chain launch");
             br.done();
             g_launches++;
+        }
+        if (!on_device && c + 1 < nchunks) { // behind this chunk's launches: from pageable memory it holds the host
+            const std::vector<int32_t> next = piece_ends(c + 1);
+            for (int p = 0; p < (int)next.size(); ++p)
+                if (int rc = issue_copy(c + 1, p, p == 0 ? 0 : next[p - 1], next[p])) return rc;
         }
         if (ctx->out_tro)
             CK(cudaMemcpyAsync(ctx->host_tro.data() + (size_t)s0 * M * N, ctx->tro[slot].p,
