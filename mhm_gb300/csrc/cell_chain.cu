@@ -88,7 +88,28 @@ cudaError_t launch_cell_chain_fused(const FusedCellArgs &f, int hl, bool lean, i
     return cudaGetLastError();
 }
 
-// occ = resident blocks per SM the kernel's registers are sized for (4, 6, 8)
+// The register variant of a launch nobody chose one for: the fewest waves of
+// blocks, then the fewest blocks an SM -- more registers shorten a step, another
+// wave repeats all of them.  With 7 or 8 horizons 8 blocks' planes do not fit an
+// SM's shared memory.  3 horizons, 48 steps, 4 / 6 / 8 blocks: 62,500 cells 0.51 /
+// 0.61 / 0.68 ms, 99,856 cells 0.90 / 0.71 / 0.79, 160,000 cells 1.31 / 1.23 /
+// 1.42, 250,000 cells 1.83 / 1.78 / 1.71; 6 horizons, 24 steps: 144,400 cells
+// 0.75 / 0.88 / 0.68, 640,000 cells 3.10 / 2.83 / 2.86, 1e6 cells 4.65 / 4.24 /
+// 4.21; 8 horizons 1e6 cells 5.57 / 5.07 / 5.56.
+static int cell_chain_occ(const CellArgs &a, int H)
+{
+    const int64_t n = (int64_t)a.n_cells * a.n_members;
+    int best = 4;
+    int64_t best_waves = INT64_MAX;
+    for (int occ = 4; occ <= (H <= 6 ? 8 : 6); occ += 2) {
+        const int64_t per_wave = (int64_t)152 * 128 * occ, waves = (n + per_wave - 1) / per_wave;
+        if (waves < best_waves) best = occ, best_waves = waves;
+    }
+    return best;
+}
+
+// occ = resident blocks per SM the kernel's registers are sized for (4, 6, 8; 0:
+// by the rule above)
 cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
 {
     if (H < 1 || H > kMaxHorizons) return cudaErrorInvalidValue;
@@ -99,6 +120,7 @@ cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
     // 3.40 / 5.69, 160,000 cells 11.9 / 10.3 / 14.3).
     if (cell_chain_fits_small(a)) return launch_cell_chain_small(a, s);
     if (a.flux_aet || a.out.n_planes > 0) return launch_cell_chain_variant<3, true>(a, H, s);
+    if (occ == 0) occ = cell_chain_occ(a, H);
     switch (occ) {
     case 6: return launch_cell_chain_o6(a, H, s);
     case 8: return launch_cell_chain_o8(a, H, s);

@@ -196,7 +196,7 @@ struct mhm_ctx {
     // of n_lai entries, its parameters in lai_series [M][3][n_lai][N]
     int32_t lai_mode = 0, n_lai = 0;
     DevBuf<double> lai_series;
-    int32_t cell_occ = 4;  // cell-chain register variant: resident blocks per SM (4, 6, 8)
+    int32_t cell_occ = 0;  // cell-chain register variant: resident blocks per SM (4, 6, 8; 0: by the launch's size)
     int32_t cell_small = 1; // launches of few cells take the kernel of cell_chain_small.cu
     int32_t chunk_cap = 0; // most time steps per chunk (0: the device-memory budget decides)
     // routing case 2: per-member routing time step [s] and the link lengths
@@ -1975,7 +1975,7 @@ int mhm_set_launch_config(mhm_ctx *ctx, const mhm_launch_config *cfg)
 int mhm_get_launch_config(mhm_ctx *ctx, mhm_launch_config *cfg)
 {
     if (!ctx || !cfg) return MHM_ERR_INVALID;
-    cfg->cell_blocks_per_sm = ctx->cell_occ;
+    cfg->cell_blocks_per_sm = ctx->cell_occ ? ctx->cell_occ : 4;
     cfg->route_sub_steps = ctx->route_sub;
     cfg->chunk_steps = ctx->chunk_cap;
     cfg->route_cluster = ctx->route_cluster;

@@ -152,3 +152,27 @@ def test_outputs_small_equals_one_thread_a_cell(monkeypatch, flags, H, nr, nc, p
     assert res[0][6].shape[0] == 3 and np.isfinite(res[0][6]).all() and np.any(res[0][6] != 0.0)
     for i, (a, b) in enumerate(zip(*res)):
         assert np.array_equal(a, b), i
+
+
+@pytest.mark.parametrize("H,nr,nc", [(2, 278, 280), (2, 278, 281), (3, 417, 281), (7, 278, 281), (6, 624, 250)])
+def test_default_variant_by_size(H, nr, nc):
+    """around one wave of 4, 6 and 8 blocks an SM: the variant a launch takes by
+    its size gives the results of a chosen one"""
+    from mhm_gb300.model import MhmGpu
+    dom = synth.make_domain(nr, nc, H, l11_factor=8, seed=2)
+    p = _params(dom, 0, 3)
+    f = _forcing(dom, 0, True, 12)
+    res = []
+    for occ in (None, 4):
+        g = MhmGpu(dom)
+        try:
+            if occ:
+                g.set_launch_config(cell_blocks_per_sm=occ)
+            assert g.get_launch_config()["cell_blocks_per_sm"] == 4
+            g.prepare(p, synth.ROUTING_PARAMS_DEFAULT)
+            g.set_meteo(1, **f)
+            res.append([g.run(1, 12)] + [g.get_state()[k] for k in STATES])
+        finally:
+            g.close()
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
