@@ -101,18 +101,23 @@ __device__ bool wait_step(const RouteArgs &a, const longlong2 *p, uint64_t id, u
 // qOUT, then the Muskingum recurrence.
 //
 // What bounds it: the tick, a chain of dependent FP64 operations (64 cycles
-// each on this GPU, three plus one per upstream link) and a block barrier; a
-// chunk of T steps takes T ticks plus the length of the river.  So everything a
+// each on this GPU, three plus one per upstream link), of the instructions
+// around them -- two warps wait for each in turn, so addresses move with the
+// step instead of being computed from it (107 -> about 80 a tick: 36 nodes, 2,160
+// steps 1.35 -> 1.02 ms) -- and a block barrier; a chunk of T steps takes T
+// ticks plus the length of the river.  So everything a
 // tick reads is already on the chip: outflows pass from node to node through a
 // ring in shared memory, a node's own runoff and the outflows of other blocks
 // are fetched a round of S ticks ahead.  A block exports the outflow of its
 // pieces' last nodes to device memory, step by step.  Measured (one chunk of
 // 240 steps): 62,500 nodes, 1,478 deep, 2.1 ms; the same on a 1,458-deep grid
-// 2.2-2.4 ms; 576 nodes 0.20 ms.  A launch (or a cluster barrier) per wavefront
+// 2.1-2.4 ms; 576 nodes 0.19 ms.  A launch (or a cluster barrier) per wavefront
 // of all nodes, whose loads all came from device memory, took 16.1, 27.9 and
 // 0.69 ms.  64 nodes a block: with 32 a 576-node network takes 0.24 ms (more
 // hand-overs), with 128 the deep one gains nothing (the FP64 pipe of the SM is
-// shared by more warps a tick).  S = 8 covers a device-memory load; S = 4 hands
+// shared by more warps a tick).  Two threads a node, one for
+// the sum and one for the recurrence, take 7-14 % longer: the hand-over costs
+// more than it takes off the chain.  S = 8 covers a device-memory load; S = 4 hands
 // over sooner, 6-8 % faster where the river is longer than the chunk and as
 // much slower where it is not.
 //
@@ -198,15 +203,34 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
     auto fetch = [&](int r) {
         if (add_qout) {
             const int t0 = r * S - lag, h0 = (r & 1) * S;
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(&own_q[h0][tid]);
+            auto get = [&](int j, const double *src) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + j * kRouteBlock * 8), "l"(src) : "memory");
+            };
+            if (t0 >= 0 && t0 + S <= nT && a.rdiv == 1) {
+                if (bc_ok(BC_ROUTE_QOUT, t0 + S - 1, a.n_qsteps)) {
+                    const double *src = qo + (size_t)t0 * L;
 #pragma unroll
-            for (int j = 0; j < S; ++j) {
-                const int t = t0 + j;
-                if ((unsigned)t < (unsigned)nT) {
+                    for (int j = 0; j < S; ++j, src += L) get(j, src);
+                }
+            } else if (t0 >= 0 && t0 + S <= nT) {
+                const int row = t0 / a.rdiv;
+                int left = (row + 1) * a.rdiv - t0; // steps that take this row
+                if (bc_ok(BC_ROUTE_QOUT, (t0 + S - 1) / a.rdiv, a.n_qsteps)) {
+                    const double *src = qo + (size_t)row * L;
+#pragma unroll
+                    for (int j = 0; j < S; ++j) {
+                        get(j, src);
+                        if (--left == 0) src += L, left = a.rdiv;
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < S; ++j) {
+                    const int t = t0 + j;
+                    if ((unsigned)t >= (unsigned)nT) continue;
                     const int row = a.rdiv == 1 ? t : t / a.rdiv;
-                    if (!bc_ok(BC_ROUTE_QOUT, row, a.n_qsteps)) continue;
-                    const unsigned dst = (unsigned)__cvta_generic_to_shared(&own_q[h0 + j][tid]);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(qo + (size_t)row * L)
-                                 : "memory");
+                    if (bc_ok(BC_ROUTE_QOUT, row, a.n_qsteps)) get(j, qo + (size_t)row * L);
                 }
             }
         }
@@ -232,6 +256,9 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     };
+    // a node's steps follow one another from 0, so its pointers move with them
+    longlong2 *out_t = out;
+    uint64_t id_t = a.done0;
     // one tick; `k` its number, `i` its row of the ring
     auto tick = [&](int k, int i) {
         const double *row = ring[(i - 1) & (2 * S - 1)];
@@ -243,9 +270,14 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
             q = q + v1;
             if (nu_warp > 2) q = q + v2;
             if (nu_warp > 3) {
+                q = q + row[up[3]];
+                if (nu_warp > 4) {
+                    q = q + row[up[4]];
+                    if (nu_warp > 5) {
 #pragma unroll
-                for (int u = 3; u < kRouteUps; ++u)
-                    if (u < nu_warp) q = q + row[up[u]];
+                        for (int u = 5; u < kRouteUps; ++u) q = q + row[up[u]];
+                    }
+                }
             }
         }
         if (hub_warp && hub >= 0) {
@@ -265,10 +297,13 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
         double qtr = keep + c2 * (q - qtin1);
         if (cut_warp) qtr = hm_sel(cut, 0.0, qtr);
         ring[i][tid] = qtr;
-        if (out_warp && out) put_step(out + t, qtr, a.done0 + (uint64_t)t);
+        if (out_warp && out) put_step(out_t, qtr, id_t);
+        ++out_t;
+        ++id_t;
         qtr1 = qtr;
         qtin1 = q;
-        if (qmod_warp && keep_qmod) qm[(size_t)t * L] = q; // L11_qMod = (0 + Qmod) / real(rout_loop = 1)
+        if (qmod_warp && keep_qmod) *qm = q; // L11_qMod = (0 + Qmod) / real(rout_loop = 1)
+        qm += L;
     };
     if (tid < 2 * S) ring[tid][kZero] = 0.0;
 #pragma unroll
