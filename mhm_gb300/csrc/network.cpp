@@ -42,13 +42,15 @@ bool build_route_network(int32_t L, int32_t n_outlets, const int32_t *net_perm, 
     // upstream nodes of each node in rank order of their links, and the nodes
     // in rank order of their own link (sinks last): upstream before downstream
     std::vector<std::vector<int32_t>> ups(L);
-    std::vector<int32_t> topo, topo_of(L, -1);
+    std::vector<int32_t> topo, topo_of(L, -1), above(L, 0); // above: links of the longest river into a node
     for (int32_t r = 0; r < nl; ++r) {
         const int32_t i = net_perm[r] - 1, f = from_n[i] - 1;
         ups[to_n[i] - 1].push_back(f);
+        above[to_n[i] - 1] = std::max(above[to_n[i] - 1], above[f] + 1);
         topo_of[f] = (int32_t)topo.size();
         topo.push_back(f);
     }
+    o.depth = *std::max_element(above.begin(), above.end());
     for (int32_t v = 0; v < L; ++v)
         if (down[v] < 0) {
             topo_of[v] = (int32_t)topo.size();

@@ -25,6 +25,7 @@ constexpr int kRouteBlock = 64;
 struct RouteNetwork {
     int32_t n_nodes = 0, n_links = 0;
     int32_t n_blocks = 0, n_exports = 0;
+    int32_t depth = 0;                 // links of the longest river
     std::vector<int32_t> pos_of_node;  // [n_nodes] 0-based node -> position
     std::vector<int32_t> node_of_pos;  // [n_nodes]
     std::vector<int8_t> pos_flags;     // bit0 is link, bit1 adds its own qOUT
