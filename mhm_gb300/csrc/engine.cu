@@ -242,7 +242,7 @@ struct mhm_batch {
     int64_t *h_item0 = nullptr;
     size_t cap_ctx = 0, cap_tiles = 0;
     int64_t rounds = 0, tiles_total = 0;
-    int32_t occ = 8; // register variant of the fused launch: 4 or 8 resident blocks per SM
+    int32_t occ = 0; // register variant of the fused launch: 4 or 8 resident blocks per SM (0: by its tiles)
     std::string err;
 };
 
@@ -3058,7 +3058,11 @@ int mhm_batch_run_members(mhm_batch *b, int32_t n, mhm_ctx *const *ctxs, const i
     f.tile_item0 = b->tile_item0.p;
     f.n_tiles = (int32_t)n_tiles;
     f.queue = b->queue.p;
-    if (cudaError_t e = launch_cell_chain_fused(f, hl, lean, b->occ, b->stream))
+    // 4 blocks an SM, with more registers, while the tiles fill them once and little
+    // more (120 steps, 4 / 8 blocks: 448 tiles 1.77 / 2.31 ms, 646 tiles 2.84 / 3.23,
+    // 886 tiles 2.90 / 2.46, 1,201 tiles 3.91 / 3.77, 2,294 tiles 6.69 / 5.96)
+    const int occ = b->occ ? b->occ : n_tiles <= 684 ? 4 : 8;
+    if (cudaError_t e = launch_cell_chain_fused(f, hl, lean, occ, b->stream))
         return bfail(MHM_ERR_CUDA, std::string("fused cell chain: ") + cudaGetErrorString(e));
     g_launches++;
     if (cudaEventRecord(b->ev_done, b->stream) != cudaSuccess) return bfail(MHM_ERR_CUDA, "event");

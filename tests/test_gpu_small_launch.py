@@ -176,3 +176,36 @@ def test_default_variant_by_size(H, nr, nc):
             g.close()
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("occ", ["4", "8", None])
+def test_fused_variants(monkeypatch, occ):
+    """both register variants of the fused launch, and the one it takes by its
+    tiles, give the results of each context's own launch"""
+    import torch
+    from mhm_gb300.model import MhmBatch, MhmGpu
+    if occ:
+        monkeypatch.setenv("MHM_FUSED_OCC", occ)
+    doms = [synth.make_domain(9, 17, 2, l11_factor=3, seed=1), synth.make_domain(13, 11, 6, l11_factor=2, seed=2)]
+    fs = [{k: torch.from_numpy(v).cuda() for k, v in synth.make_forcing(d, 60, seed=4).items()} for d in doms]
+    res = []
+    for fused in (True, False):
+        gs, qs = [MhmGpu(d) for d in doms], [np.zeros((1, len(d.gauge_node), 60)) for d in doms]
+        try:
+            for g, d, f in zip(gs, doms, fs):
+                g.prepare(_params(d, 0, 7), synth.ROUTING_PARAMS_DEFAULT)
+                g.set_meteo(1, **f, on_device=True)
+            t0 = [np.array([1], np.int32)] * 2
+            if fused:
+                MhmBatch().run_members(gs, t0, 60, qs)
+            else:
+                for g, q in zip(gs, qs):
+                    g.run_members_async(t0[0], 60, q)
+            for g in gs:
+                g.sync()
+            res.append(qs + [g.get_state()[k] for g in gs for k in STATES])
+        finally:
+            for g in gs:
+                g.close()
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
