@@ -380,8 +380,8 @@ def run_gpu(args) -> dict:
                      "kernel": "cell_chain_kernel<6>", "alg_bytes_per_launch": alg_bytes,
                      "launch_ms": per_launch_s * 1e3, "peak_source": "of measured (MEASURED_PEAKS.json hbm_gbs)"
                      if peaks else "of fallback",
-                     "binding_roof": "the FP64 pipe (roofline_fp64.pipe_frac) and instruction issue "
-                                     "(roofline_issue); HBM is not the limit"},
+                     "binding_roof": "latency at 32 warps per SM; the FP64 pipe (roofline_fp64.pipe_frac) and "
+                                     "instruction issue (roofline_issue) about half busy; HBM is not the limit"},
         "roofline_fp64": fp64_line,
         "roofline_issue": issue_line,
         "kernel_time_ms": {"cell_chain": t_cell, "runoff_acc": t_acc, "routing": t_rt,
