@@ -190,8 +190,9 @@ __device__ __noinline__ Uptake uptake_general(bool feddes, double aet, double sm
 
 // The part of a cell's step above the soil -- meteo, canopy, snow and the sealed
 // bucket -- which depends on the forcing and on its own states only.  KEEP keeps
-// the meteo of a daily forcing row from hour to hour (it changes with the row,
-// the month and day or night) at the price of registers.
+// the meteo of a daily forcing row from step to step (it changes with the row,
+// the month and day or night, Hargreaves-Samani PET with the day too: a row is
+// 24 steps, and above one hour a step several days) at the price of registers.
 template <bool LEAN, bool KEEP = false> struct Surface {
     // states
     double interc, snow, seal;
@@ -322,7 +323,8 @@ template <bool LEAN, bool KEEP = false> struct Surface {
         bool fresh = true;
         if constexpr (KEEP) {
             const int day = key << 1 | (si.dflags & SF_ISDAY);
-            fresh = a.is_hourly || a.w_pet || f != cur_f || day != cur_day;
+            fresh = a.is_hourly || a.w_pet || f != cur_f || day != cur_day ||
+                    (!LEAN && a.proc_pet == 1 && si.doy != cur_doy);
             cur_f = f;
             cur_day = day;
         }
