@@ -276,13 +276,15 @@ int mhm_run_members_async(mhm_ctx *ctx, const int32_t *member_tt0, int32_t n_ste
  * in (variant, sub-chunk) order. */
 int mhm_autotune(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *occ_out, int32_t *sub_out, double *ms_out);
 
-/* How a context launches its work (no counterpart in the reference).  A context
- * whose configuration was never set or tuned chooses the first two by the size of
- * a launch and the depth of its network, and reports 4 and 8; launches of few
- * cells take a kernel of their own whatever the variant. */
+/* How a context launches its work (no counterpart in the reference).  The first
+ * two are 0 in a context where they were never set or tuned; what was read can be
+ * written back.  Launches of few cells take a kernel of their own whatever the
+ * variant. */
 typedef struct mhm_launch_config {
-    int32_t cell_blocks_per_sm; /* cell-chain register variant: 4, 6 or 8 resident blocks per SM */
-    int32_t route_sub_steps;    /* steps the routing fetches ahead at a time, 1..16 (4, or 8 above 4) */
+    int32_t cell_blocks_per_sm; /* cell-chain register variant: 4, 6 or 8 resident blocks per SM; 0: by the
+                                   size of each launch */
+    int32_t route_sub_steps;    /* steps the routing fetches ahead at a time, 1..16 (4, or 8 above 4); 0: by
+                                   the depth of the network and the length of the chunk */
     int32_t chunk_steps;        /* most time steps per chunk (0: the device-memory budget decides) */
     int32_t route_cluster;      /* 0, 4, 8 or 16: accepted and reported back; a chunk's routing is one
                                    launch for each */

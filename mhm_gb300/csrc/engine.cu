@@ -1963,10 +1963,11 @@ int mhm_snapshot_load(mhm_ctx *ctx, int32_t slot, int32_t member) { return snaps
 int mhm_set_launch_config(mhm_ctx *ctx, const mhm_launch_config *cfg)
 {
     if (!ctx || !cfg) return MHM_ERR_INVALID;
-    if (cfg->cell_blocks_per_sm != 4 && cfg->cell_blocks_per_sm != 6 && cfg->cell_blocks_per_sm != 8)
-        return fail(ctx, MHM_ERR_INVALID, "cell_blocks_per_sm must be 4, 6 or 8");
-    if (cfg->route_sub_steps < 1 || cfg->route_sub_steps > 16)
-        return fail(ctx, MHM_ERR_INVALID, "route_sub_steps must be 1..16");
+    if (cfg->cell_blocks_per_sm != 0 && cfg->cell_blocks_per_sm != 4 && cfg->cell_blocks_per_sm != 6 &&
+        cfg->cell_blocks_per_sm != 8)
+        return fail(ctx, MHM_ERR_INVALID, "cell_blocks_per_sm must be 0, 4, 6 or 8");
+    if (cfg->route_sub_steps < 0 || cfg->route_sub_steps > 16)
+        return fail(ctx, MHM_ERR_INVALID, "route_sub_steps must be 0..16");
     if (cfg->chunk_steps < 0) return fail(ctx, MHM_ERR_INVALID, "chunk_steps must be >= 0");
     if (cfg->route_cluster != 0 && cfg->route_cluster != 4 && cfg->route_cluster != 8 && cfg->route_cluster != 16)
         return fail(ctx, MHM_ERR_INVALID, "route_cluster must be 0, 4, 8 or 16");
@@ -1981,8 +1982,8 @@ int mhm_set_launch_config(mhm_ctx *ctx, const mhm_launch_config *cfg)
 int mhm_get_launch_config(mhm_ctx *ctx, mhm_launch_config *cfg)
 {
     if (!ctx || !cfg) return MHM_ERR_INVALID;
-    cfg->cell_blocks_per_sm = ctx->cell_occ ? ctx->cell_occ : 4;
-    cfg->route_sub_steps = ctx->route_sub ? ctx->route_sub : 8;
+    cfg->cell_blocks_per_sm = ctx->cell_occ;
+    cfg->route_sub_steps = ctx->route_sub;
     cfg->chunk_steps = ctx->chunk_cap;
     cfg->route_cluster = ctx->route_cluster;
     return MHM_OK;
@@ -2160,7 +2161,7 @@ int mhm_autotune(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *occ_out, i
     mhm_launch_config b{};
     const int rc = mhm_autotune_ex(ctx, tt0, n_steps, 0, nullptr, &b, ms_out);
     if (occ_out) *occ_out = b.cell_blocks_per_sm;
-    if (sub_out) *sub_out = b.route_sub_steps;
+    if (sub_out) *sub_out = b.route_sub_steps ? b.route_sub_steps : 8; // without routing there is none to choose
     return rc;
 }
 

@@ -40,6 +40,19 @@ class MhmError(RuntimeError):
     pass
 
 
+# launch knobs that can be left to each launch, and what they are for a launch of moderate size
+_BY_LAUNCH = {"cell_blocks_per_sm": 4, "route_sub_steps": 8}
+
+
+def _launch_config_dict(cfg) -> dict:
+    out = {n: getattr(cfg, n) for n in ("cell_blocks_per_sm", "route_sub_steps", "chunk_steps", "route_cluster")}
+    auto = tuple(n for n in _BY_LAUNCH if out[n] == 0)
+    out.update({n: _BY_LAUNCH[n] for n in auto})
+    if auto:
+        out["by_launch"] = auto
+    return out
+
+
 class MhmGpu:
     """One basin (optionally with n_members parameter sets) on one GPU."""
 
@@ -416,19 +429,26 @@ class MhmGpu:
         best = _lib.LaunchConfig()
         self._check(self.L.mhm_autotune_ex(self.ctx, tt0, n_steps, ch.size, _i(ch) if ch.size else None,
                                            C.byref(best), _d(ms)), "mhm_autotune_ex")
-        return {"cell_blocks_per_sm": best.cell_blocks_per_sm, "route_sub_steps": best.route_sub_steps,
-                "chunk_steps": best.chunk_steps, "route_cluster": best.route_cluster, "trial_ms": ms.tolist()}
+        return {**_launch_config_dict(best), "trial_ms": ms.tolist()}
 
-    def set_launch_config(self, cell_blocks_per_sm: int = 4, route_sub_steps: int = 8, chunk_steps: int = 0,
-                          route_cluster: int = 0):
+    def set_launch_config(self, cell_blocks_per_sm: int = 0, route_sub_steps: int = 0, chunk_steps: int = 0,
+                          route_cluster: int = 0, by_launch=()):
+        """mhm_set_launch_config; cell_blocks_per_sm and route_sub_steps left out, 0
+        or named in `by_launch` are chosen launch by launch."""
         cfg = _lib.LaunchConfig(cell_blocks_per_sm, route_sub_steps, chunk_steps, route_cluster)
+        for name in by_launch:
+            if name not in _BY_LAUNCH:
+                raise ValueError(f"by_launch: {name}")
+            setattr(cfg, name, 0)
         self._check(self.L.mhm_set_launch_config(self.ctx, C.byref(cfg)), "mhm_set_launch_config")
 
     def get_launch_config(self) -> dict:
+        """The configuration, as set_launch_config(**...) takes it back.  A knob that
+        is chosen launch by launch is named in "by_launch" and stands there with
+        the value of a launch of moderate size."""
         cfg = _lib.LaunchConfig()
         self._check(self.L.mhm_get_launch_config(self.ctx, C.byref(cfg)), "mhm_get_launch_config")
-        return {"cell_blocks_per_sm": cfg.cell_blocks_per_sm, "route_sub_steps": cfg.route_sub_steps,
-                "chunk_steps": cfg.chunk_steps, "route_cluster": cfg.route_cluster}
+        return _launch_config_dict(cfg)
 
     def snapshot_alloc(self, n_slots: int):
         self._check(self.L.mhm_snapshot_alloc(self.ctx, n_slots), "mhm_snapshot_alloc")
