@@ -273,7 +273,9 @@ int mhm_run_members_async(mhm_ctx *ctx, const int32_t *member_tt0, int32_t n_ste
  * 16), restoring all members' states before each trial and after the
  * last, and keeps the fastest for the context's later runs.  Needs the
  * forcing for those steps.  ms_out (may be NULL) receives the 9 trial times
- * in (variant, sub-chunk) order. */
+ * in (variant, sub-chunk) order; combinations that launch the same kernels
+ * (rounds of 8 and 16; every variant where a launch has few cells) are timed
+ * once. */
 int mhm_autotune(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *occ_out, int32_t *sub_out, double *ms_out);
 
 /* How a context launches its work (no counterpart in the reference).  The first
@@ -301,10 +303,10 @@ int mhm_get_launch_config(mhm_ctx *ctx, mhm_launch_config *cfg);
  * configuration kept. */
 int mhm_autotune_ex(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t n_chunk_choices,
                     const int32_t *chunk_choices, mhm_launch_config *best_out, double *ms_out);
-/* Times n_steps from tt0 with route_cluster 0, 4, 8 and 16 in that order
- * (states restored afterwards; ms_out, may be NULL: 4 trial times); the
- * fastest is kept and written to *cluster_out (may be NULL).  All four launch
- * the same kernel.  Contexts without routing keep 0. */
+/* route_cluster 0, 4, 8 and 16 are the same launch: times n_steps from tt0 once
+ * (states restored afterwards), writes that time to the four of ms_out (may be
+ * NULL; -1 in contexts without routing) and the context's value, which stays, to
+ * *cluster_out (may be NULL). */
 int mhm_autotune_route(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *cluster_out, double *ms_out);
 
 /* Device-resident restart states: n_slots snapshot slots per context (each

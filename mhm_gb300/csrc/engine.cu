@@ -26,6 +26,7 @@
 
 namespace mhm {
 cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s);
+bool cell_chain_fits_small(const CellArgs &a);
 cudaError_t launch_steps_fill(StepInfo *steps, int64_t tt0, int32_t n, int32_t jul_start, int32_t timestep,
                               int32_t stride, int32_t lai_mode, cudaStream_t s);
 cudaError_t launch_runoff_acc(const AccArgs &a, cudaStream_t s);
@@ -2089,23 +2090,36 @@ int mhm_autotune_ex(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t n_chunk_
     // loading of each kernel variant and buffers of each chunk length
     std::vector<int> warm;
     for (int c = 0; c < nc; ++c)
-        for (int j = 0; j < 3; ++j) warm.push_back(c * 9 + j);     // (4, sub) for each chunk length
+        for (int j = 0; j < 2; ++j) warm.push_back(c * 9 + j);     // (4, sub) for each chunk length
     warm.push_back(3);                                            // (6, 4)
     warm.push_back(6);                                            // (8, 4)
     const int nw = (int)warm.size();
+    // trials that would launch the same kernels as an earlier one have its time:
+    // rounds of 16 steps are rounds of 8, and few cells take one kernel whatever
+    // the variant
+    CellArgs shape{};
+    shape.n_cells = ctx->N;
+    shape.n_members = ctx->M;
+    shape.n_horizons = ctx->H;
+    shape.proc_sm = ctx->proc_sm;
+    shape.proc_pet = ctx->proc_pet;
+    shape.small_ok = ctx->cell_small;
+    const bool one_variant = cell_chain_fits_small(shape);
+    std::vector<double> ms_of(n_trials, -1.0);
     for (int trial = -nw; rc == MHM_OK && trial < n_trials; ++trial) {
         const int ti = trial < 0 ? warm[trial + nw] : trial;
         const int c = ti / 9, v = ti % 9;
+        const int same = c * 9 + (one_variant ? 0 : v / 3 * 3) + std::min(v % 3, 1);
+        if (same != ti || (!rout && v % 3 != 0)) {
+            if (trial >= 0) ms_of[trial] = rout || v % 3 == 0 ? ms_of[same] : -1.0;
+            continue;
+        }
         ctx->cell_occ = occs[v / 3];
         ctx->route_sub = rout ? subs[v % 3] : sub0;
         ctx->chunk_cap = caps[c];
-        if (!rout && v % 3 != 0) {
-            if (trial >= 0 && ms_out) ms_out[trial] = -1.0;
-            continue;
-        }
         float ms = 0.f;
         if ((rc = ts.trial(tt0, n_steps, &ms))) break;
-        if (trial >= 0 && ms_out) ms_out[trial] = ms;
+        if (trial >= 0) ms_of[trial] = ms;
         if (trial >= 0 && ms < best) {
             best = ms;
             best_occ = ctx->cell_occ;
@@ -2113,6 +2127,7 @@ int mhm_autotune_ex(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t n_chunk_
             best_cap = ctx->chunk_cap;
         }
     }
+    if (ms_out && rc == MHM_OK) std::copy(ms_of.begin(), ms_of.end(), ms_out);
     ctx->cell_occ = rc == MHM_OK ? best_occ : occ0;
     ctx->route_sub = rc == MHM_OK ? best_sub : sub0;
     ctx->chunk_cap = rc == MHM_OK ? best_cap : cap0;
@@ -2127,30 +2142,15 @@ int mhm_autotune_route(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *clus
     if (!ctx || n_steps < 1) return MHM_ERR_INVALID;
     ON_CTX_DEVICE(ctx);
     if (int rc = mhm_sync(ctx)) return rc;
-    const int32_t modes[4] = {0, 4, 8, 16};
-    const int32_t mode0 = ctx->route_cluster;
     int rc = MHM_OK;
-    int32_t best_mode = mode0;
-    if (ctx->proc_rout >= 1 && ctx->L > 1) {
+    float ms = -1.f;
+    if (ctx->proc_rout >= 1 && ctx->L > 1) { // every value is the same launch: one time stands for the four
         TuneScope ts(ctx);
         rc = ts.copy_states(true);
-        float best = 1e30f;
-        for (int trial = -4; rc == MHM_OK && trial < 4; ++trial) { // one untimed pass over the modes first
-            ctx->route_cluster = modes[trial < 0 ? trial + 4 : trial];
-            float ms = 0.f;
-            if ((rc = ts.trial(tt0, n_steps, &ms))) break;
-            if (trial < 0) continue;
-            if (ms_out) ms_out[trial] = ms;
-            if (ms < best) {
-                best = ms;
-                best_mode = ctx->route_cluster;
-            }
-        }
-        ctx->route_cluster = rc == MHM_OK ? best_mode : mode0;
+        for (int i = 0; rc == MHM_OK && i < 2; ++i) rc = ts.trial(tt0, n_steps, &ms); // untimed once
         rc = ts.finish(rc);
-    } else if (ms_out) {
-        for (int i = 0; i < 4; ++i) ms_out[i] = -1.0;
     }
+    for (int i = 0; ms_out && rc == MHM_OK && i < 4; ++i) ms_out[i] = ms;
     if (cluster_out) *cluster_out = ctx->route_cluster;
     return rc;
 }

@@ -413,8 +413,8 @@ class MhmGpu:
         return out
 
     def autotune_route(self, tt0: int, n_steps: int) -> dict:
-        """mhm_autotune_route: route_cluster 0, 4, 8, 16 timed (all launch the
-        same kernel)."""
+        """mhm_autotune_route: route_cluster 0, 4, 8 and 16 are the same launch; its
+        time, four times, and the context's value."""
         cl = C.c_int32()
         ms = np.zeros(4)
         self._check(self.L.mhm_autotune_route(self.ctx, tt0, n_steps, C.byref(cl), _d(ms)), "mhm_autotune_route")
