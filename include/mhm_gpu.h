@@ -40,7 +40,7 @@ extern "C" {
 #define MHM_ERR_INVALID (-1)     /* bad argument or shape */
 #define MHM_ERR_CUDA (-2)        /* CUDA runtime error or no device */
 #define MHM_ERR_OOM (-3)         /* device allocation failed */
-#define MHM_ERR_TIMEOUT (-4)     /* a bounded device wait ran out */
+#define MHM_ERR_TIMEOUT (-4)     /* a bounded device wait ran out: see mhm_sync */
 #define MHM_ERR_NAN (-5)         /* non-finite state or forcing detected */
 #define MHM_ERR_UNSUPPORTED (-6) /* process option not implemented */
 #define MHM_ERR_BOUNDS (-7)      /* bounds-checked build: an index taken from data was out of range */
@@ -247,7 +247,12 @@ int mhm_run(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gauge);
  * valid until mhm_sync returns; state access and the set-up calls
  * synchronise first.  Per-step outputs (mhm_enable_outputs) need mhm_run. */
 int mhm_run_async(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gauge);
-/* Wait for all enqueued work of the context. */
+/* Wait for all enqueued work of the context.  MHM_ERR_TIMEOUT: a bounded wait of
+ * the routing ran out.  The discharge of every run enqueued since the last
+ * mhm_sync (q_gauge is filled all the same), its outputs and the context's states
+ * are then void; the context stays usable from states that are set anew
+ * (mhm_init_states, mhm_set_state, mhm_snapshot_load).  mhm_run and every call
+ * that synchronises first report it the same way, once. */
 int mhm_sync(mhm_ctx *ctx);
 /* Without waiting: *done = 1 if all work enqueued so far has completed on
  * the device (mhm_sync then returns at once and finishes the host side:
