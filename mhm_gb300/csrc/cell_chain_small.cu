@@ -2,6 +2,7 @@
 // idle: few cells, so that the time of a call is the latency of a step, not the
 // throughput of the SMs.
 #include "cell_chain_impl.cuh"
+#include "small_launch.h"
 
 namespace mhm {
 
@@ -37,7 +38,7 @@ __device__ __forceinline__ void bar_sync(int id, int threads)
 // FLUX, aggregated outputs or per-step fluxes: one more warp adds up what the
 // others post of a step while they work on the next.
 template <int H, bool LEAN, bool FLUX>
-__global__ void __launch_bounds__(32 * (H + 2 + FLUX), 1024 / (32 * (H + 2 + FLUX)))
+__global__ void __launch_bounds__(32 * (H + 2 + FLUX), small_blocks_per_sm(H, FLUX))
     cell_chain_small_kernel(const CellArgs a)
 {
     __shared__ double s_sm[H][32], s_fr[H][32], s_st[H][32], s_sms[H][32];
@@ -305,20 +306,14 @@ template <bool LEAN, bool FLUX> static cudaError_t launch_small(const CellArgs &
     }
 }
 
-// Up to 180,000 warps' lanes (cells times H + 2): where the blocks no longer fit
-// the GPU at once (96 steps, this kernel / one thread a cell: 1 horizon, 40,000
-// cells 0.45 / 0.67 ms, 62,500 cells 0.80 / 0.76; 3 horizons, 25,600 cells 0.51 /
-// 0.78, 40,000 cells 0.81 / 0.88, 62,500 cells 1.25 / 0.99; 6 horizons, 16,384
-// cells 0.61 / 0.96, 25,600 cells 1.01 / 1.10, 40,000 cells 1.48 / 1.25).  With
-// outputs, whose warp takes more off the other kernel's chain, up to 235,000
-// (cells times H + 3; 14 or more planes: 1 horizon, 3,600 cells 0.27 / 0.72,
-// 62,500 cells 1.20 / 1.91; 3 horizons, 3,600 cells 0.38 / 0.95, 25,600 cells
-// 1.00 / 1.14, 40,000 cells 1.31 / 1.31, 52,900 cells 1.75 / 1.34; 6 horizons,
-// 9,216 cells 0.68 / 1.35, 25,600 cells 1.33 / 1.59, 40,000 cells 1.98 / 1.83).
 bool cell_chain_fits_small(const CellArgs &a)
 {
+    int dev = 0, sms = 0;
+    if (!a.small_ok || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return false;
     const bool flux = a.flux_aet || a.out.n_planes > 0;
-    return a.small_ok && (int64_t)a.n_cells * a.n_members * (a.n_horizons + 2 + flux) <= (flux ? 235000 : 180000);
+    return small_launch(a.n_horizons, cell_chain_lean(a), flux, (int64_t)a.n_cells * a.n_members, sms);
 }
 
 cudaError_t launch_cell_chain_small(const CellArgs &a, cudaStream_t s)
