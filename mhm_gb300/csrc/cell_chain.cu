@@ -78,11 +78,9 @@ cudaError_t launch_cell_chain_fused(const FusedCellArgs &f, int hl, bool lean, i
         return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, nb = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    int nb = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, block, smem)) != cudaSuccess) return e;
-    const int64_t wave = (int64_t)(nb < 1 ? 1 : nb) * sms;
+    const int64_t wave = (int64_t)(nb < 1 ? 1 : nb) * device_sms();
     const unsigned grid = (unsigned)(f.n_tiles < wave ? f.n_tiles : wave);
     k<<<grid, block, smem, s>>>(f);
     return cudaGetLastError();
@@ -99,10 +97,11 @@ cudaError_t launch_cell_chain_fused(const FusedCellArgs &f, int hl, bool lean, i
 static int cell_chain_occ(const CellArgs &a, int H)
 {
     const int64_t n = (int64_t)a.n_cells * a.n_members;
+    const int sms = device_sms();
     int best = 4;
     int64_t best_waves = INT64_MAX;
     for (int occ = 4; occ <= (H <= 6 ? 8 : 6); occ += 2) {
-        const int64_t per_wave = (int64_t)152 * 128 * occ, waves = (n + per_wave - 1) / per_wave;
+        const int64_t per_wave = (int64_t)sms * 128 * occ, waves = (n + per_wave - 1) / per_wave;
         if (waves < best_waves) best = occ, best_waves = waves;
     }
     return best;

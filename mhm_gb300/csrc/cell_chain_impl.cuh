@@ -532,6 +532,17 @@ __device__ __forceinline__ void out_close(const OutArgs &o, double *acc, size_t 
     cnt = 0;
 }
 
+// SMs of the current device: the launch rules count in waves of blocks.  152 (a
+// GB300's), should the runtime not say.
+__host__ inline int device_sms()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return 152;
+    return sms;
+}
+
 __host__ inline bool cell_chain_lean(const CellArgs &a)
 {
     return (a.proc_pet == 0 || a.proc_pet == -1) && (a.proc_sm == 1 || a.proc_sm == 4);
@@ -889,7 +900,7 @@ __host__ __device__ constexpr bool member_tiles(int64_t n_members) { return n_me
 // cells, 96 steps: 144 ms with 128 threads, 130 with 256, 131 with 512).  With
 // 6 horizons the horizon loop is most of the step, and smaller blocks wait less
 // at the barriers (1e6 cells, 96 steps: 16.5 / 17.1 / 18.0 ms).
-constexpr int64_t kWideItems = (int64_t)152 * 8 * 128 * 4;
+inline int64_t wide_items(int sms) { return (int64_t)sms * 8 * 128 * 4; }
 constexpr bool wide_blocks(int H, int MINB, bool FLUX) { return H <= 3 && MINB >= 6 && !FLUX; }
 
 template <int H, int MINB, bool FLUX, bool LEAN, int B>
@@ -968,7 +979,7 @@ cudaError_t launch_cell_chain_b(const CellArgs &a, cudaStream_t s)
 template <int MINB, bool FLUX, bool LEAN>
 cudaError_t launch_cell_chain_h(const CellArgs &a, int H, cudaStream_t s)
 {
-    const bool wide = (int64_t)a.n_cells * a.n_members >= kWideItems;
+    const bool wide = wide_blocks(H, MINB, FLUX) && (int64_t)a.n_cells * a.n_members >= wide_items(device_sms());
     switch (H) {
 #define MHM_CASE(HH)                                                                                               \
     case HH:                                                                                                       \

@@ -308,12 +308,8 @@ template <bool LEAN, bool FLUX> static cudaError_t launch_small(const CellArgs &
 
 bool cell_chain_fits_small(const CellArgs &a)
 {
-    int dev = 0, sms = 0;
-    if (!a.small_ok || cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return false;
     const bool flux = a.flux_aet || a.out.n_planes > 0;
-    return small_launch(a.n_horizons, cell_chain_lean(a), flux, (int64_t)a.n_cells * a.n_members, sms);
+    return a.small_ok && small_launch(a.n_horizons, cell_chain_lean(a), flux, (int64_t)a.n_cells * a.n_members, device_sms());
 }
 
 cudaError_t launch_cell_chain_small(const CellArgs &a, cudaStream_t s)
