@@ -3,6 +3,7 @@
 // for 6 and 8 resident blocks per SM live in cell_chain_o6.cu / _o8.cu, the
 // kernel of small launches in cell_chain_small.cu.
 #include "cell_chain_impl.cuh"
+#include "launch_rules.h"
 
 namespace mhm {
 
@@ -101,7 +102,7 @@ static int cell_chain_occ(const CellArgs &a, int H)
     int best = 4;
     int64_t best_waves = INT64_MAX;
     for (int occ = 4; occ <= (H <= 6 ? 8 : 6); occ += 2) {
-        const int64_t per_wave = (int64_t)sms * 128 * occ, waves = (n + per_wave - 1) / per_wave;
+        const int64_t waves = waves_of(n, sms, occ);
         if (waves < best_waves) best = occ, best_waves = waves;
     }
     return best;
@@ -112,13 +113,11 @@ static int cell_chain_occ(const CellArgs &a, int H)
 cudaError_t launch_cell_chain(const CellArgs &a, int H, int occ, cudaStream_t s)
 {
     if (H < 1 || H > kMaxHorizons) return cudaErrorInvalidValue;
-    // per-step fluxes or aggregated outputs: one register variant.  With 3 blocks
-    // an SM they hold what a step adds up; with 4 some of it goes through local
-    // memory, with 2 a large launch lacks warps (3 horizons, 14 planes, 240 steps,
-    // 4 / 3 / 2 blocks: 3,600 cells 2.76 / 2.56 / 2.50 ms, 40,000 cells 3.62 /
-    // 3.40 / 5.69, 160,000 cells 11.9 / 10.3 / 14.3).
     if (cell_chain_fits_small(a)) return launch_cell_chain_small(a, s);
-    if (a.flux_aet || a.out.n_planes > 0) return launch_cell_chain_variant<3, true>(a, H, s);
+    if (a.flux_aet || a.out.n_planes > 0) // per-step fluxes or aggregated outputs
+        return flux_blocks_per_sm((int64_t)a.n_cells * a.n_members, device_sms()) == 4
+                   ? launch_cell_chain_variant<4, true>(a, H, s)
+                   : launch_cell_chain_variant<3, true>(a, H, s);
     if (occ == 0) occ = cell_chain_occ(a, H);
     switch (occ) {
     case 6: return launch_cell_chain_o6(a, H, s);

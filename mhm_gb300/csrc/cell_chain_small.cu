@@ -2,7 +2,7 @@
 // idle: few cells, so that the time of a call is the latency of a step, not the
 // throughput of the SMs.
 #include "cell_chain_impl.cuh"
-#include "small_launch.h"
+#include "launch_rules.h"
 
 namespace mhm {
 
