@@ -1633,6 +1633,7 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         r.n_qsteps = nT / F;
         r.n_blocks = ctx->net.n_blocks;
         r.n_exports = ctx->net.n_exports;
+        r.n_hubs = (int32_t)ctx->net.hub_ptr.size() - 1;
         r.blk_ptr = ctx->blk_ptr.p;
         r.blk_lag = ctx->blk_lag.p;
         r.ext_ptr = ctx->ext_ptr.p;

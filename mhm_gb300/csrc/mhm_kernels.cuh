@@ -174,11 +174,11 @@ struct AccArgs {
     double TST;                  // HourSecs * routing timestep
     const double *tro;           // [n_steps][M][n_cells]
     const double *l1_area;       // [n_cells]
-    const int32_t *node_cell_ptr; // [n_nodes+1] by level position
+    const int32_t *node_cell_ptr; // [n_nodes+1] by routing position
     const int32_t *node_cells;    // ascending L1 index per node
     const int32_t *pos_l11_l1;    // [n_nodes] 0-based L1 cell of the node (!map_flag)
     const double *pos_area;       // [n_nodes] L11 area by position
-    double *qout;                 // [M][n_steps][n_nodes] by level position
+    double *qout;                 // [M][n_steps][n_nodes] by routing position
     const int32_t *member_step0;  // member mode: < 0 marks an idle member (skipped)
 };
 
@@ -187,6 +187,7 @@ struct AccArgs {
 struct RouteArgs {
     int32_t n_nodes, n_members, n_steps;
     int32_t n_blocks, n_exports;
+    int32_t n_hubs;             // nodes with more than kRouteUps upstream links
     const int32_t *blk_ptr, *blk_lag, *ext_ptr, *ext_export, *ext_lag, *pos_lag, *pos_export, *hub_ptr, *hub_ups;
     const int16_t *pos_ups;     // [n_nodes][kRouteUps]
     const int8_t *pos_flags;    // bit0: is link (has C1/C2), bit1: add qOUT, bit2: the link's routed

@@ -20,7 +20,7 @@ namespace mhm {
 
 // L11_runoff_acc, src/mRM/mo_mrm_pre_routing.f90:77-143: per (step, member,
 // node) the area-weighted sum of its L1 cells in ascending cell order, then
-// *1000/TST.  Output indexed by routing-level position.
+// *1000/TST.  Output indexed by routing position.
 __global__ void __launch_bounds__(256) runoff_acc_kernel(const AccArgs a)
 {
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -95,6 +95,43 @@ __device__ bool wait_step(const RouteArgs &a, const longlong2 *p, uint64_t id, u
     return true;
 }
 
+// The upstream links of a node with more of them than a thread keeps (none on a D8
+// grid), by the lanes that are in this tick together: for each such node among them
+// (`hub` >= 0) every lane reads the step of one link, and the next link's while these
+// are added to the node's sum q one after another in their order.  Read by the node's
+// own thread, each link was a trip to the L2 (a node with 2,000 of them, 240 steps:
+// 161 ms; 56 ms where all blocks met after each step; 34 so).
+__device__ __forceinline__ double add_hubs(const RouteArgs &a, const longlong2 *qx, int hub, int t, double q, bool &bad)
+{
+    const unsigned act = __activemask();
+    const int lane = threadIdx.x & 31, n_act = __popc(act), rank = __popc(act & ((1u << lane) - 1));
+    for (unsigned hubs = __ballot_sync(act, hub >= 0); hubs != 0; hubs &= hubs - 1) {
+        const int src = __ffs((int)hubs) - 1, h = __shfl_sync(act, hub, src), th = __shfl_sync(act, t, src);
+        const int u0 = __ldg(a.hub_ptr + h), u1 = __ldg(a.hub_ptr + h + 1);
+        const uint64_t id = a.done0 + (uint64_t)th;
+        const longlong2 *p = nullptr;
+        uint64_t v = 0, got = id; // a lane without a link: adding +0 changes nothing
+        auto fetch = [&](int u) {
+            const int x = u < u1 ? __ldg(a.hub_ups + u) : -1;
+            p = x >= 0 && bc_ok(BC_ROUTE_UP, x, a.n_exports) ? qx + (size_t)x * a.qx_stride + th : nullptr;
+            v = 0;
+            got = id;
+            if (p) get_step(p, v, got);
+        };
+        double sum = __shfl_sync(act, q, src);
+        fetch(u0 + rank);
+        for (int u = u0; u < u1; u += n_act) {
+            if (got != id && !bad) bad = !wait_step(a, p, id, v);
+            const double mine = __longlong_as_double((long long)v);
+            __syncwarp(act);
+            fetch(u + n_act + rank);
+            for (unsigned m = act; m != 0; m &= m - 1) sum = sum + __shfl_sync(act, mine, __ffs((int)m) - 1);
+        }
+        if (lane == src) q = sum;
+    }
+    return q;
+}
+
 // One block of the network for one member: a thread per node, a step per tick,
 // each node `lag` ticks behind the block's first.  L11_routing body,
 // src/mRM/mo_mrm_routing.f90:435-478: ((0 + qTR(up_1)) + qTR(up_2) + ...) +
@@ -125,7 +162,10 @@ __device__ bool wait_step(const RouteArgs &a, const longlong2 *p, uint64_t id, u
 // which a pair waits only on pairs taken before it.  So whatever the number of
 // resident blocks, the oldest running one waits on nothing unfinished and the
 // launch ends; the limit in wait_step only guards against a defect.
-template <int S>
+//
+// HUB: the network has nodes whose upstream links are read by add_hubs; another
+// instantiation, so that its registers are not every network's.
+template <int S, bool HUB>
 __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs a)
 {
     // by tick: the outflows of the block's nodes, then of the series it takes,
@@ -161,7 +201,7 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
         const int4 w = __ldg(reinterpret_cast<const int4 *>(a.pos_ups) + pos);
         const int v[kRouteUps] = {(int16_t)w.x, w.x >> 16, (int16_t)w.y, w.y >> 16,
                                   (int16_t)w.z, w.z >> 16, (int16_t)w.w, w.w >> 16};
-        if (v[0] == -2) {
+        if (HUB && v[0] == -2) {
             hub = v[1] + (v[2] << 15);
         } else {
 #pragma unroll
@@ -186,7 +226,7 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
     // never -0), so all lanes of a warp add as many links as the longest list;
     // likewise the +0 runoff of a node that adds none.
     const int nu_warp = (int)__reduce_max_sync(~0u, (unsigned)nu);
-    const bool hub_warp = __any_sync(~0u, hub >= 0), cut_warp = __any_sync(~0u, cut);
+    const bool hub_warp = HUB && __any_sync(~0u, hub >= 0), cut_warp = __any_sync(~0u, cut);
     const bool out_warp = __any_sync(~0u, ex >= 0), qmod_warp = __any_sync(~0u, keep_qmod);
     const int lag_hi = (int)__reduce_max_sync(~0u, (unsigned)lag);
     const int lag_lo = (int)__reduce_min_sync(~0u, own ? (unsigned)lag : 0xffffu);
@@ -280,15 +320,8 @@ __global__ void __launch_bounds__(kRouteBlock) route_flow_kernel(const RouteArgs
                 }
             }
         }
-        if (hub_warp && hub >= 0) {
-            const int u1 = __ldg(a.hub_ptr + hub + 1);
-            for (int u = __ldg(a.hub_ptr + hub); u < u1; ++u) {
-                const int x = __ldg(a.hub_ups + u);
-                if (!bc_ok(BC_ROUTE_UP, x, a.n_exports)) continue;
-                uint64_t v = 0;
-                if (!bad) bad = !wait_step(a, qx + (size_t)x * a.qx_stride + t, a.done0 + (uint64_t)t, v);
-                q = q + __longlong_as_double((long long)v);
-            }
+        if constexpr (HUB) {
+            if (hub_warp) q = add_hubs(a, qx, hub, t, q, bad);
         }
         q = q + qo_t;
         // 0 + (-0) is +0: the sum starts at netNode_qTIN(:, IT) = 0
@@ -509,9 +542,10 @@ cudaError_t launch_route_flow(const RouteArgs &a, int round, cudaStream_t s)
 {
     if (a.n_members < 1 || a.n_steps < 1) return cudaSuccess;
     const unsigned grid = (unsigned)(a.n_blocks * a.n_members);
-    if (round <= 4) route_flow_kernel<4><<<grid, kRouteBlock, 0, s>>>(a);
-    else if (round <= 16) route_flow_kernel<8><<<grid, kRouteBlock, 0, s>>>(a);
-    else return cudaErrorInvalidValue;
+    if (round > 16) return cudaErrorInvalidValue;
+    const auto kernel = a.n_hubs > 0 ? (round <= 4 ? route_flow_kernel<4, true> : route_flow_kernel<8, true>)
+                                     : (round <= 4 ? route_flow_kernel<4, false> : route_flow_kernel<8, false>);
+    kernel<<<grid, kRouteBlock, 0, s>>>(a);
     return cudaGetLastError();
 }
 
