@@ -457,7 +457,16 @@ struct Ground {
         }
     }
 
-    // L1_total_runoff, mo_runoff.f90:248-274
+    // The unsealed share as total() takes it: NaN for an infinite sealed fraction,
+    // whose product with a sealed runoff of +0, left out there, is NaN, as is that
+    // of a positive one less the infinite unsealed part.
+    static __device__ __forceinline__ double share(double fsealed)
+    {
+        const bool finite = (hm_hi(hm_d2b(fsealed)) & 0x7ff00000u) != 0x7ff00000u;
+        return hm_sel(finite, 1.0 - fsealed, hm_b2d(0x7ff8000000000000ULL));
+    }
+
+    // L1_total_runoff, mo_runoff.f90:248-274; `fnotsealed` from share()
     __device__ __forceinline__ double total(double fnotsealed, double runoff_sealed, double fsealed) const
     {
         double q = base + slow;
@@ -601,7 +610,7 @@ __device__ __forceinline__ void cell_chain_item(const CellArgs &a, const int m, 
     if (tb < 3) s_wet[tb] = 0;
     __syncthreads();
     const bool feddes = LEAN || (a.proc_sm == 1 || a.proc_sm == 4);
-    const double fsealed = par(P_FSEALED), fnotsealed = 1.0 - fsealed;
+    const double fsealed = par(P_FSEALED), fnotsealed = 1.0 - fsealed, share = Ground::share(fsealed);
     const double jarvis = LEAN ? 0.0 : par(P_JARVIS);
     const uint64_t r_jarvis = LEAN ? 0 : hm_recip_of(jarvis);
     Surface<LEAN> sf;
@@ -843,7 +852,7 @@ __device__ __forceinline__ void cell_chain_item(const CellArgs &a, const int m, 
                 a.flux_loss[fo] = fnotsealed * (gd.perc - gd.perc * gd.karst);
             }
         }
-        const double q_total = gd.total(fnotsealed, sf.runoff_sealed, fsealed);
+        const double q_total = gd.total(share, sf.runoff_sealed, fsealed);
         tro[(size_t)t * out_stride] = q_total;
         nonfin |= hm_abs_bits(hm_d2b(q_total)) + kExpOne;
         if constexpr (FLUX) {

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(32 * (H + 2 + FLUX), small_blocks_per_sm(H, FL
     } else if (part == 0) { // soil
         Ground gd;
         gd.load(a, P, S);
-        const double fsealed = par(P_FSEALED), fnotsealed = 1.0 - fsealed;
+        const double fsealed = par(P_FSEALED), share = Ground::share(fsealed);
         bool frac_bounded = true; // every horizon's runoff fraction is in [0, 1]
         for (int h = 0; h < H; ++h) {
             const double sms = par(P_HORIZON + H + h);
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(32 * (H + 2 + FLUX), small_blocks_per_sm(H, FL
             bar_sync(2, below); // the soil moisture of the step
             if (active) {
                 gd.step(infil);
-                const double q_total = gd.total(fnotsealed, s_rsealed[t & 1][lane], fsealed);
+                const double q_total = gd.total(share, s_rsealed[t & 1][lane], fsealed);
                 tro[(size_t)t * out_stride] = q_total;
                 chk(q_total);
                 if constexpr (FLUX) {
