@@ -258,7 +258,7 @@ def run_gpu(args) -> dict:
     torch.cuda.synchronize()
     stream = torch.cuda.ExternalStream(g.stream, device=device)
     g.set_meteo(1, pre, temp, pet, on_device=True)
-    tune = None if args.no_autotune else g.autotune(1, chunk)   # register variant x routing sub-chunk
+    tune = None if args.no_autotune else g.autotune(1, chunk)   # register variant x routing round
 
     G = len(dom.gauge_node)
     qbufs = [np.zeros((1, G, chunk)) for _ in range(2)]
@@ -416,7 +416,7 @@ def run_ensemble(args, device, plain_members: int = 8) -> dict:
     horizons, L0 = L1/4, 256 parameter sets drawn uniformly within the
     namelist bounds, hourly.  Batched: one context holds all 256 members
     (device MPR for all of them in one call, one cell-chain launch per chunk
-    over member x cell, routing of all members per wavefront tick).  Plain:
+    over member x cell, one routing launch for all members).  Plain:
     the one-parameter-set drop-in, members one after another (each with its
     own MPR and run), timed on `plain_members` members.  Both advance every
     member by the same chunks of 240 steps; throughput counts member x cell x

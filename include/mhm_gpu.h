@@ -278,7 +278,7 @@ int mhm_run_members_async(mhm_ctx *ctx, const int32_t *member_tt0, int32_t n_ste
  * 16), restoring all members' states before each trial and after the
  * last, and keeps the fastest for the context's later runs.  Needs the
  * forcing for those steps.  ms_out (may be NULL) receives the 9 trial times
- * in (variant, sub-chunk) order; combinations that launch the same kernels
+ * in (variant, round) order; combinations that launch the same kernels
  * (rounds of 8 and 16; every variant where a launch has few cells) are timed
  * once. */
 int mhm_autotune(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t *occ_out, int32_t *sub_out, double *ms_out);
@@ -300,11 +300,11 @@ int mhm_set_launch_config(mhm_ctx *ctx, const mhm_launch_config *cfg);
 int mhm_get_launch_config(mhm_ctx *ctx, mhm_launch_config *cfg);
 /* mhm_autotune over one more knob, the time-chunk length: each of the
  * n_chunk_choices chunk lengths (0 = as the memory budget allows; at most 8)
- * is tried with every register variant and routing sub-chunk.  A run is
+ * is tried with every register variant and routing round.  A run is
  * split into chunks whose routing overlaps the next chunk's cell chain, so
  * shorter chunks trade launches for overlap.  n_chunk_choices = 0 keeps the
  * context's chunk length.  ms_out (may be NULL) receives 9 trial times per
- * chunk length, in (chunk length, variant, sub-chunk) order; best_out the
+ * chunk length, in (chunk length, variant, round) order; best_out the
  * configuration kept. */
 int mhm_autotune_ex(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, int32_t n_chunk_choices,
                     const int32_t *chunk_choices, mhm_launch_config *best_out, double *ms_out);

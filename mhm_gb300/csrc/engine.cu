@@ -1671,9 +1671,9 @@ static int run_enqueue(mhm_ctx *ctx, int32_t tt0, int32_t n_steps, double *q_gau
         {
             Bracket br(ctx, 2, rs);
             // a river longer than the chunk: most of the time is the way from block to
-            // block, which shorter rounds make faster (1,458 links, 240 steps: 2.11 / 2.36
-            // ms with rounds of 4 / 8; 56 links: 0.266 / 0.260; 27 links, 720 steps 0.52 /
-            // 0.475)
+            // block, which shorter rounds make faster (1,458 links, 240 steps: 1.86 / 2.25
+            // ms with rounds of 4 / 8; 27 links, 720 steps 0.432 / 0.424; 8 links, 2,160
+            // steps 0.98 / 0.93)
             const int sub = ctx->route_sub ? ctx->route_sub : ctx->net.depth > n_rsteps ? 4 : 8;
             CK(launch_route_flow(r, sub, rs), "route launch");
             ctx->route_ticket0 += (uint32_t)(r.n_blocks * r.n_members);

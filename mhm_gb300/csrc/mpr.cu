@@ -6,8 +6,8 @@
 // functions, the depth-weighted horizon properties, the root fractions and
 // the Ks variabilities.  So the first kernel evaluates them once per pair and
 // member into a small table (tens of rows instead of millions of L0 cells);
-// the second kernel gives every L1 cell one thread that walks its L0
-// sub-cells in the reference's column-major block order and forms the
+// the second kernel gives every L1 cell a lane in each of H + 4 warps that
+// walk its L0 sub-cells in the reference's column-major block order and forms the
 // arithmetic and harmonic means from table rows and the few per-cell inputs
 // (slope rank, aspect, LAI, geology), writing the member's effective
 // parameters in place.  The per-cell values are the same IEEE operations on

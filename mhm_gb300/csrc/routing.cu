@@ -140,23 +140,23 @@ __device__ __forceinline__ double add_hubs(const RouteArgs &a, const longlong2 *
 // What bounds it: the tick, a chain of dependent FP64 operations (64 cycles
 // each on this GPU, three plus one per upstream link), of the instructions
 // around them -- two warps wait for each in turn, so addresses move with the
-// step instead of being computed from it (107 -> about 80 a tick: 36 nodes, 2,160
-// steps 1.35 -> 1.02 ms) -- and a block barrier; a chunk of T steps takes T
+// step instead of being computed from it, and what few networks need is an
+// instantiation of its own (107 -> 75 a tick: 36 nodes, 2,160 steps 1.35 -> 0.93 ms) -- and a block barrier; a chunk of T steps takes T
 // ticks plus the length of the river.  So everything a
 // tick reads is already on the chip: outflows pass from node to node through a
 // ring in shared memory, a node's own runoff and the outflows of other blocks
 // are fetched a round of S ticks ahead.  A block exports the outflow of its
 // pieces' last nodes to device memory, step by step.  Measured (one chunk of
-// 240 steps): 62,500 nodes, 1,478 deep, 2.1 ms; the same on a 1,458-deep grid
-// 2.1-2.4 ms; 576 nodes 0.19 ms.  A launch (or a cluster barrier) per wavefront
+// 240 steps): 62,500 nodes, 1,478 deep, 1.9 ms; the same on a 1,458-deep grid
+// 1.9 ms; 576 nodes 0.17 ms.  A launch (or a cluster barrier) per wavefront
 // of all nodes, whose loads all came from device memory, took 16.1, 27.9 and
 // 0.69 ms.  64 nodes a block: with 32 a 576-node network takes 0.24 ms (more
 // hand-overs), with 128 the deep one gains nothing (the FP64 pipe of the SM is
 // shared by more warps a tick).  Two threads a node, one for
 // the sum and one for the recurrence, take 7-14 % longer: the hand-over costs
 // more than it takes off the chain.  S = 8 covers a device-memory load; S = 4 hands
-// over sooner, 6-8 % faster where the river is longer than the chunk and as
-// much slower where it is not.
+// over sooner, 15-17 % faster where the river is longer than the chunk and up to
+// 5 % slower where it is not.
 //
 // Blocks take (network block, member) pairs from a counter, in an order in
 // which a pair waits only on pairs taken before it.  So whatever the number of

@@ -400,7 +400,7 @@ class MhmGpu:
         self._check(self.L.mhm_set_output_weights(self.ctx, member, tt, _d(fs), _d(sm)), "mhm_set_output_weights")
 
     def autotune(self, tt0: int, n_steps: int, route: bool = True) -> dict:
-        """Pick the fastest cell-chain register variant and routing sub-chunk
+        """Pick the fastest cell-chain register variant and routing round
         by timing n_steps from tt0 (states restored afterwards); with `route`
         also autotune_route."""
         occ = C.c_int32()
@@ -421,7 +421,7 @@ class MhmGpu:
         return {"route_cluster": cl.value, "route_trial_ms": ms.tolist()}
 
     def autotune_ex(self, tt0: int, n_steps: int, chunk_choices=()) -> dict:
-        """The autotuner over register variant x routing sub-chunk x time-chunk
+        """The autotuner over register variant x routing round x time-chunk
         length (mhm_autotune_ex); returns the configuration kept."""
         ch = np.ascontiguousarray(chunk_choices, np.int32)
         nc = max(1, ch.size)
